@@ -8,6 +8,7 @@
 //                            restarts, primal weight, phases and certification
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -231,6 +232,9 @@ void convert_data(Problem& P, VecSet<V>& vs, cudaStream_t s) {
     }
 }
 
+template <class M, class V>
+void init_resident_attrs();
+
 // Kernels whose dynamic shared memory exceeds the 48 KB default opt in.
 void init_kernel_attrs() {
     static std::once_flag once;
@@ -249,6 +253,10 @@ void init_kernel_attrs() {
         set_smem(k_dplr_expand<double, 1>, expand_smem_bytes<double, 1>(kMaxRank));
         set_smem(k_dplr_expand<double, 2>, expand_smem_bytes<double, 2>(kMaxRank));
         set_smem(k_spmv_q2<double, double>, spmv_smem_bytes<2, double>());
+        init_resident_attrs<float, float>();
+        init_resident_attrs<__nv_bfloat16, float>();
+        init_resident_attrs<float, double>();
+        init_resident_attrs<double, double>();
     });
 }
 
@@ -386,6 +394,7 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     P->red_arrivals.reset(1);
     GB_CUDA(cudaMemsetAsync(P->red_arrivals.get(), 0, sizeof(unsigned), s));
     P->st.reset(count);
+    P->phase_flags.reset(count + 1);
     GB_CUDA(cudaMemsetAsync(P->st.get(), 0, sizeof(SolveState) * count, s));
 
     // schedules (host, from the row-length histogram, per instance) and transpose
@@ -510,9 +519,8 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     prebuild_graphs(*P, opt);
     tr.mark("fp32 copies+graphs");
     P->st_host = static_cast<SolveState*>(host_alloc(sizeof(SolveState) * count));
-    P->phase_flags_host = static_cast<int*>(host_alloc(sizeof(int) * count));
+    P->phase_flags_host = static_cast<int*>(host_alloc(sizeof(int) * (count + 1)));
     tr.mark("pinned state");
-    P->phase_flags.reset(count);
     GB_CUDA(cudaMemcpyAsync(P->scal_host.data(), sc, sizeof(double) * P->scal_host.size(), cudaMemcpyDeviceToHost, s));
     GB_CUDA(cudaStreamSynchronize(s));
     GB_CUDA(cudaGetLastError());
@@ -627,9 +635,24 @@ EvalArgs<M, V> eval_args(Problem& P, VecSet<V>& vs, const V* x, const V* y, int 
     return a;
 }
 
+// Row blocks the streaming kernels of a body run: the partial phase's, else
+// those of the instances that are not iterated on chip, else all (na < 0).
+struct StreamBlocks {
+    const RowBlock *a = nullptr, *t = nullptr;
+    int na = -1, nt = -1;
+};
+template <class M, class V>
+StreamBlocks stream_blocks(const Problem& P) {
+    const ResPlan& R = P.res[sizeof(V) == 8];
+    if (P.list_level == level_index<M, V>()) return {P.list_a.get(), P.list_t.get(), P.list_na, P.list_nt};
+    if (R.any()) return {R.list_a.get(), R.list_t.get(), R.list_na, R.list_nt};
+    return {};
+}
+
 // Arguments of the two kernels of the k-th iteration inside a body (buffers by parity).
 template <class M, class V>
-void iteration_args(Problem& P, VecSet<V>& vs, int k, PrimalArgs<M, V>& pa, DualArgs<M, V>& da) {
+void iteration_args(Problem& P, VecSet<V>& vs, int k, PrimalArgs<M, V>& pa, DualArgs<M, V>& da,
+                    const StreamBlocks& sb = {}) {
     const V* xin = (k & 1) ? vs.x1.get() : vs.x0.get();
     V* xout = (k & 1) ? vs.x0.get() : vs.x1.get();
     const V* yin = (k & 1) ? vs.y1.get() : vs.y0.get();
@@ -638,11 +661,11 @@ void iteration_args(Problem& P, VecSet<V>& vs, int k, PrimalArgs<M, V>& pa, Dual
                           P.has_q ? vs.qx.get() : nullptr, xout, vs.xbar.get(), vs.sumx.get(), P.st.get()};
     da = DualArgs<M, V>{P.A.view<M>(), vs.xbar.get(), yin, vs.lo.get(), vs.hi.get(), yout, vs.sumy.get(),
                         P.st.get()};
-    if (P.list_level == level_index<M, V>()) {  // a phase of some instances only
-        pa.AT.blocks = P.list_t.get();
-        pa.AT.nb = P.list_nt;
-        da.A.blocks = P.list_a.get();
-        da.A.nb = P.list_na;
+    if (sb.na >= 0) {
+        pa.AT.blocks = sb.t;
+        pa.AT.nb = sb.nt;
+        da.A.blocks = sb.a;
+        da.A.nb = sb.na;
     }
 }
 
@@ -666,12 +689,285 @@ void launch_dual(const DualArgs<M, V>& da, cudaStream_t s) {
         launch_pdl(k_dual<M, V>, da.A.nb, kThreads, spmv_seg_smem_bytes<V>(), s, da);
 }
 
+// ---------------------------------------------------------------- instances iterated on chip
+// GANIT_B200_RESIDENT=0 streams every instance (same FP32 bits).
+bool resident_enabled() {
+    static const bool on = [] {
+        const char* v = std::getenv("GANIT_B200_RESIDENT");
+        return v == nullptr || std::string(v) != "0";
+    }();
+    return on;
+}
+
+template <class M, class V>
+void init_resident_attrs() {
+    auto set = [](auto kernel) {
+        set_smem(kernel, kResMaxSmem);
+        GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    };
+    set(k_resident<M, V, 256>);
+    set(k_resident<M, V, 512>);
+    set(k_resident<M, V, 1024>);
+}
+
+template <class M, class V>
+auto resident_kernel(int threads) {
+    return threads == 256 ? k_resident<M, V, 256> : threads == 512 ? k_resident<M, V, 512> : k_resident<M, V, 1024>;
+}
+
+// Launch configuration of a class (attr must outlive it).
+inline cudaLaunchConfig_t resident_config(const ResClass& c, cudaLaunchAttribute* attr, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c.nctas);
+    cfg.blockDim = dim3(c.threads);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = c.cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <class M>
+const M* resident_values(const ResPlan& R);
+template <>
+const float* resident_values<float>(const ResPlan& R) { return R.val32.get(); }
+template <>
+const double* resident_values<double>(const ResPlan& R) { return R.val64.get(); }
+template <>
+const __nv_bfloat16* resident_values<__nv_bfloat16>(const ResPlan& R) { return R.valbf.get(); }
+
+// check_every iterations of a class's instances (iterate in buffer 0; the
+// result goes where the streaming kernels leave theirs).
+template <class M, class V>
+void launch_resident(Problem& P, VecSet<V>& vs, const ResClass& c, int ce, cudaStream_t s) {
+    const ResPlan& R = P.res[sizeof(V) == 8];
+    const bool odd = (ce & 1) != 0;
+    ResArgs<M, V> a{R.cta.get() + c.cta0, R.slices.get(), R.idx.get(), resident_values<M>(R), R.col_at.get(),
+                    R.row_at.get(), vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(),
+                    odd ? vs.y1.get() : vs.y0.get(), vs.sumx.get(), vs.sumy.get(), vs.c.get(), vs.l.get(),
+                    vs.u.get(), vs.lo.get(), vs.hi.get(), P.st.get(), P.phase_flags.get() + P.count, ce, c.cluster};
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = resident_config(c, attr, s);
+    GB_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel<M, V>(c.threads), a));
+}
+
+// Packed values of matrix type M (made on first use; the structure is there).
+template <class M, class V>
+void ensure_resident_values(Problem& P) {
+    ResPlan& R = P.res[sizeof(V) == 8];
+    if (!R.any()) return;
+    cudaStream_t s = P.stream;
+    auto pack = [&](auto& buf, auto src) {
+        if (buf.get()) return;
+        buf.reset(static_cast<size_t>(R.pairs) * 64);
+        GB_CUDA(cudaMemsetAsync(buf.get(), 0, buf.size() * sizeof(*buf.get()), s));
+        const int gt = elem_grid(P.n, P.sms), ga = elem_grid(P.m, P.sms);
+        k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), R.slot_t.get(), R.at.get(), buf.get());
+        k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), R.slot_a.get(), R.at.get(), buf.get());
+    };
+    if constexpr (std::is_same<M, double>::value) pack(R.val64, [](const DevMat& A) { return A.val64.get(); });
+    else if constexpr (std::is_same<M, float>::value) pack(R.val32, [](const DevMat& A) { return A.val32.get(); });
+    else pack(R.valbf, [](const DevMat& A) { return A.valbf.get(); });
+    GB_CUDA(cudaGetLastError());
+}
+
+// Which instances run on chip with vectors of type V (index w), in clusters
+// of what size, and their packed structure.  An instance qualifies when its
+// rows are all STREAM rows, its positions fit 16 bits and a cluster of at
+// most 16 CTAs holds it.  The cluster size follows its share of the GPU's
+// SMs by work (a lone LP spreads over 16, an instance of a large batch takes
+// the fewest CTAs that hold it), but no CTA gets fewer than kResMinSlices
+// slices, where the barrier outweighs the work.
+constexpr int kResMinSlices = 4;
+template <class V>
+void ensure_resident(Problem& P) {
+    constexpr int w = sizeof(V) == 8;
+    constexpr size_t sm = sizeof(V);  // FP64 vectors: sized for the FP64 matrix
+    ResPlan& R = P.res[w];
+    if (R.built) return;
+    R.built = true;
+    R.resident.assign(P.count, 0);
+    if (P.has_q || !resident_enabled()) return;
+    const DevSchedule& sa = P.A.template sched_for<V>();
+    const DevSchedule& st = P.AT.template sched_for<V>();
+    const long long most = static_cast<long long>(kResMaxCluster * kResMaxSmem / (2 * (2 + sm)));
+    std::vector<std::array<ResHist, 2>> hist;
+    std::vector<int> who;
+    std::vector<double> work;
+    double total = 0.0;
+    for (int k = 0; k < P.count; ++k) {
+        const int n = P.col_off[k + 1] - P.col_off[k], m = P.row_off[k + 1] - P.row_off[k];
+        if (P.nnz_off[k + 1] - P.nnz_off[k] > most || std::max(n, m) + 4 * kResMaxCluster > kResMaxIndex) continue;
+        std::array<ResHist, 2> H;
+        bool ok = true;
+        for (int sd = 0; sd < 2 && ok; ++sd) {
+            const DevSchedule& sc = sd == 0 ? st : sa;
+            const int* ptr = (sd == 0 ? P.AT : P.A).host_ptr.data();
+            for (int b = sc.host_seg_block[k]; b < sc.host_seg_block[k + 1] && ok; ++b) {
+                const RowBlock& rb = sc.host_blocks[b];
+                ok = rb.kind == kStream && res_hist_rows(ptr, rb.r0, rb.r1, w ? -1 : rb.lg, H[sd]);
+            }
+            H[sd].count();
+        }
+        if (!ok) continue;
+        const double wk = static_cast<double>(H[0].pairs + H[1].pairs) + 4.0 * (H[0].slices + H[1].slices);
+        who.push_back(k);
+        hist.push_back(H);
+        work.push_back(wk);
+        total += wk;
+    }
+    if (who.empty()) return;
+    // the largest cluster that this GPU can place with the largest shared memory
+    static std::array<std::atomic<int>, 2> most_cluster{};
+    if (most_cluster[w].load() == 0) {
+        int best = 8;
+        ResClass c;
+        c.cluster = kResMaxCluster;
+        c.threads = 1024;
+        c.nctas = kResMaxCluster;
+        c.smem = kResMaxSmem;
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = resident_config(c, attr, P.stream);
+        int got = 0;
+        if (cudaOccupancyMaxActiveClusters(&got, resident_kernel<V, V>(1024), &cfg) == cudaSuccess && got > 0)
+            best = kResMaxCluster;
+        cudaGetLastError();
+        most_cluster[w].store(best);
+    }
+    const int cmax = most_cluster[w].load();
+    struct Placed {
+        int k, at;
+        ResDeal deal;
+        double work;
+        int cluster, threads;
+        size_t smem;
+    };
+    std::vector<Placed> placed;
+    for (size_t q = 0; q < who.size(); ++q) {
+        const int k = who[q];
+        const int slices = std::max(hist[q][0].slices, hist[q][1].slices);
+        const double share = work[q] * P.sms / total;
+        int C = 1;
+        while (2 * C <= cmax && 2 * C <= share && slices >= 2 * C * kResMinSlices) C *= 2;
+        Placed p{k, static_cast<int>(q), {}, work[q], 0, 0, 0};
+        const std::array<ResHist, 2>& HH = hist[q];
+        for (; C <= cmax; C *= 2) {
+            const long long pairs = HH[0].pairs + HH[1].pairs;
+            if (static_cast<size_t>(pairs) * (128 + 64 * sm) > C * kResMaxSmem) continue;  // cannot fit
+            res_deal(HH, C, p.deal);
+            p.smem = p.deal.smem(sm, sizeof(V));
+            if (p.smem <= kResMaxSmem) break;
+        }
+        if (C > cmax) continue;
+        p.cluster = C;
+        int ns = 0;
+        for (const ResCta& c : p.deal.cta) ns = std::max(ns, std::max(c.ns_t, c.ns_a));
+        p.threads = ns <= 8 ? 256 : (ns <= 16 || p.smem <= kResMaxSmem / 2 ? 512 : 1024);
+        placed.push_back(std::move(p));
+        R.resident[k] = 1;
+    }
+    if (placed.empty()) return;
+    // classes: cluster size, threads and how many CTAs an SM holds; the heaviest instances first
+    auto bucket = [](const Placed& p) { return p.smem > kResMaxSmem / 2 ? 0 : p.smem > kResMaxSmem / 4 ? 1 : 2; };
+    std::stable_sort(placed.begin(), placed.end(), [&](const Placed& x, const Placed& y) {
+        if (x.cluster != y.cluster) return x.cluster > y.cluster;
+        if (x.threads != y.threads) return x.threads > y.threads;
+        if (bucket(x) != bucket(y)) return bucket(x) < bucket(y);
+        return x.work > y.work;
+    });
+    ResTables T;
+    for (const Placed& p : placed) {
+        const bool fresh = R.classes.empty() || R.classes.back().cluster != p.cluster ||
+                           R.classes.back().threads != p.threads ||
+                           bucket(p) != bucket(placed[&p - placed.data() - 1]);
+        if (fresh) {
+            ResClass c;
+            c.cluster = p.cluster;
+            c.threads = p.threads;
+            c.cta0 = static_cast<int>(T.cta.size());
+            R.classes.push_back(c);
+        }
+        ResClass& c = R.classes.back();
+        c.nctas += p.cluster;
+        c.smem = std::max(c.smem, p.smem);
+        T.add(p.k, hist[p.at], p.deal, P.col_off[p.k], P.col_off[p.k + 1], P.row_off[p.k], P.row_off[p.k + 1]);
+    }
+    R.pairs = T.pairs;
+    cudaStream_t s = P.stream;
+    auto put = [&](auto& d, const auto& h) {
+        d.reset(std::max<size_t>(h.size(), 1));
+        d.upload(h.data(), h.size(), s);
+    };
+    put(R.cta, T.cta);
+    put(R.slices, T.slices);
+    put(R.at, T.at);
+    auto &d_t = R.sides_t, &d_a = R.sides_a;
+    put(d_t, T.sides[0]);
+    put(d_a, T.sides[1]);
+    R.idx.reset(std::max<size_t>(static_cast<size_t>(T.pairs) * 32, 1));
+    R.col_at.reset(T.positions[0]);
+    R.row_at.reset(T.positions[1]);
+    GB_CUDA(cudaMemsetAsync(R.col_at.get(), 0xff, sizeof(int) * T.positions[0], s));
+    GB_CUDA(cudaMemsetAsync(R.row_at.get(), 0xff, sizeof(int) * T.positions[1], s));
+    R.slot_t.reset(P.n);
+    R.slot_a.reset(P.m);
+    auto &pos_t = R.pos_t, &pos_a = R.pos_a;
+    auto &lg_t = R.lg_t, &lg_a = R.lg_a;
+    pos_t.reset(P.n);
+    pos_a.reset(P.m);
+    GB_CUDA(cudaMemsetAsync(R.slot_t.get(), 0xff, sizeof(int) * P.n, s));
+    GB_CUDA(cudaMemsetAsync(R.slot_a.get(), 0xff, sizeof(int) * P.m, s));
+    if (w == 0) {
+        lg_t.reset(P.n);
+        lg_a.reset(P.m);
+        k_res_row_lg<<<st.nb, kThreads, 0, s>>>(st.nb, st.blocks.get(), lg_t.get());
+        k_res_row_lg<<<sa.nb, kThreads, 0, s>>>(sa.nb, sa.blocks.get(), lg_a.get());
+    }
+    const int ns = static_cast<int>(placed.size());
+    k_res_rank<<<ns, 32, 0, s>>>(d_t.get(), P.AT.ptr.get(), lg_t.get(), R.at.get(), R.slot_t.get(), pos_t.get(),
+                                 R.col_at.get());
+    k_res_rank<<<ns, 32, 0, s>>>(d_a.get(), P.A.ptr.get(), lg_a.get(), R.at.get(), R.slot_a.get(), pos_a.get(),
+                                 R.row_at.get());
+    k_res_fill<<<static_cast<int>(T.cta.size()), kThreads, 0, s>>>(R.cta.get(), R.idx.get());
+    unsigned short* idx16 = reinterpret_cast<unsigned short*>(R.idx.get());
+    k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t.get(),
+                                                             R.at.get(), pos_a.get(), idx16);
+    k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a.get(),
+                                                             R.at.get(), pos_t.get(), idx16);
+    GB_CUDA(cudaGetLastError());
+    std::vector<RowBlock> la, lt;
+    for (int k = 0; k < P.count; ++k) {
+        if (R.resident[k]) continue;
+        la.insert(la.end(), sa.host_blocks.begin() + sa.host_seg_block[k], sa.host_blocks.begin() + sa.host_seg_block[k + 1]);
+        lt.insert(lt.end(), st.host_blocks.begin() + st.host_seg_block[k], st.host_blocks.begin() + st.host_seg_block[k + 1]);
+    }
+    R.list_na = static_cast<int>(la.size());
+    R.list_nt = static_cast<int>(lt.size());
+    put(R.list_a, la);
+    put(R.list_t, lt);
+    if (trace_enabled())
+        for (const ResClass& c : R.classes)
+            std::fprintf(stderr, "[gb trace] resident f%d: %d CTAs in clusters of %d, %d threads, %zu B\n", w ? 64 : 32,
+                         c.nctas, c.cluster, c.threads, c.smem);
+}
+
+// What a body of level <M, V> needs on chip; before its graph is captured.
+template <class M, class V>
+void prepare_resident(Problem& P) {
+    ensure_resident<V>(P);
+    ensure_resident_values<M, V>(P);
+}
+
 // One PDHG iteration (k-th inside the body) on buffers selected by parity.
 template <class M, class V>
-void launch_iteration(Problem& P, VecSet<V>& vs, int k, cudaStream_t s, long long& nl, cudaEvent_t mid = nullptr) {
+void launch_iteration(Problem& P, VecSet<V>& vs, int k, cudaStream_t s, long long& nl, cudaEvent_t mid = nullptr,
+                      const StreamBlocks& sb = {}) {
     PrimalArgs<M, V> pa;
     DualArgs<M, V> da;
-    iteration_args<M, V>(P, vs, k, pa, da);
+    iteration_args<M, V>(P, vs, k, pa, da, sb);
     if (P.has_q) launch_qx<M, V>(P, vs, pa.x, vs.qx.get(), s, nl);
     launch_primal<M, V>(pa, s);
     if (mid) GB_CUDA(cudaEventRecord(mid, s));
@@ -697,25 +993,76 @@ int launch_decide(Problem& P, EvalArgs<M, V>& ea, cudaStream_t s, bool pdl) {
     return nl;
 }
 
+// Kernels of a captured body that do not depend on one another: next() starts
+// a branch where the set began, join() makes what follows depend on the ends
+// of all of them.  Outside a capture the launches simply follow one another.
+struct Branches {
+    cudaStream_t s;
+    bool capturing = false;
+    int count = 0;
+    std::vector<cudaGraphNode_t> root, ends;
+    explicit Branches(cudaStream_t st) : s(st) { root = deps(&capturing); }
+    std::vector<cudaGraphNode_t> deps(bool* on) const {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* d = nullptr;
+        size_t k = 0;
+        GB_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &d, &k));
+        *on = status == cudaStreamCaptureStatusActive;
+        return *on ? std::vector<cudaGraphNode_t>(d, d + k) : std::vector<cudaGraphNode_t>();
+    }
+    void set(std::vector<cudaGraphNode_t>& d) {
+        GB_CUDA(cudaStreamUpdateCaptureDependencies(s, d.empty() ? nullptr : d.data(), d.size(),
+                                                    cudaStreamSetCaptureDependencies));
+    }
+    void close() {
+        bool on;
+        const std::vector<cudaGraphNode_t> d = deps(&on);
+        ends.insert(ends.end(), d.begin(), d.end());
+    }
+    void next() {
+        if (capturing && count) {
+            close();
+            set(root);
+        }
+        ++count;
+    }
+    void join() {
+        if (!capturing || count < 2) return;
+        close();
+        set(ends);
+    }
+};
+
 // Body of the phase loop: check_every iterations, KKT check, restart.
 // use_cond = 0 when the body is launched from the host loop instead of the graph.
 template <class M, class V>
 long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cudaStream_t s, int use_cond = 1) {
     VecSet<V>& vs = Level<M, V>::vs(P);
     long long nl = 0;
-    for (int k = 0; k < ce; ++k) launch_iteration<M, V>(P, vs, k, s, nl);
     const bool odd = (ce & 1) != 0;
     const V* xc = odd ? vs.x1.get() : vs.x0.get();
     const V* yc = odd ? vs.y1.get() : vs.y0.get();
+    const StreamBlocks sb = stream_blocks<M, V>(P);
+    Branches br(s);
+    for (const ResClass& c : P.res[sizeof(V) == 8].classes) {
+        br.next();
+        launch_resident<M, V>(P, vs, c, ce, s);
+        ++nl;
+    }
+    if (sb.na != 0) {
+        br.next();
+        for (int k = 0; k < ce; ++k) launch_iteration<M, V>(P, vs, k, s, nl, nullptr, sb);
+    }
+    br.join();
     if (P.has_q) launch_qx2<M, V>(P, vs, xc, s, nl);
     EvalArgs<M, V> ea = eval_args<M, V>(P, vs, xc, yc, kEvalCheck, P.has_q);
     ea.cond = cond;
     ea.use_cond = use_cond;
     const int grid = ea.A.nb + ea.AT.nb;
-    if (P.detect_unbounded && !P.has_q)  // third right-hand side of the A pass: the primal ray
-        launch_pdl(k_eval<M, V, 3, 3>, grid, kThreads, spmv_smem_bytes<3, V>(), s, ea);
-    else
-        launch_pdl(k_eval<M, V, 2, 3>, grid, kThreads, spmv_smem_bytes<3, V>(), s, ea);
+    auto eval = P.detect_unbounded && !P.has_q ? k_eval<M, V, 3, 3>  // third right-hand side of the A pass: the primal ray
+                                               : k_eval<M, V, 2, 3>;
+    if (br.count > 1) eval<<<grid, kThreads, spmv_smem_bytes<3, V>(), s>>>(ea);  // joins several branches
+    else launch_pdl(eval, grid, kThreads, spmv_smem_bytes<3, V>(), s, ea);
     nl += launch_decide<M, V>(P, ea, s, true);
     RestartArgs<V> ra{xc, yc, vs.x0.get(), vs.y0.get(), vs.xr.get(), vs.yr.get(), vs.sumx.get(), vs.sumy.get(),
                       P.n, P.m, P.icol(), P.irow(), P.st.get()};
@@ -799,9 +1146,14 @@ void prebuild_graphs(Problem& P, const gb_options* opt) {
     if (host_loop_mode() || opt->check_every <= 0) return;
     P.detect_unbounded = opt->detect_unbounded != 0;
     if (opt->precision != GB_PREC_DOUBLE) {
+        prepare_resident<float, float>(P);
         level_graph<float, float>(P, opt->check_every);
-        if (opt->precision == GB_PREC_DYNAMIC) level_graph<float, double>(P, opt->check_every);
+        if (opt->precision == GB_PREC_DYNAMIC) {
+            prepare_resident<float, double>(P);
+            level_graph<float, double>(P, opt->check_every);
+        }
     }
+    prepare_resident<double, double>(P);
     level_graph<double, double>(P, opt->check_every);
 }
 
@@ -885,12 +1237,16 @@ void set_phase_lists(Problem& P) {
     const DevSchedule& sa = P.A.template sched_for<M>();
     const DevSchedule& st = P.AT.template sched_for<M>();
     std::vector<RowBlock> la, lt;
+    int part = 0;
+    const ResPlan& R = P.res[sizeof(V) == 8];
     for (int k = 0; k < P.count; ++k) {
-        if (!P.phase_flags_host[k]) continue;
+        part += P.phase_flags_host[k];
+        if (!P.phase_flags_host[k] || R.resident[k]) continue;
         for (int b = sa.host_seg_block[k]; b < sa.host_seg_block[k + 1]; ++b) la.push_back(sa.host_blocks[b]);
         for (int b = st.host_seg_block[k]; b < st.host_seg_block[k + 1]; ++b) lt.push_back(st.host_blocks[b]);
     }
-    if (la.empty() || lt.empty() || 2 * (la.size() + lt.size()) > static_cast<size_t>(sa.nb + st.nb)) return;
+    const size_t all = R.any() ? R.list_na + R.list_nt : sa.nb + st.nb;
+    if (2 * (la.size() + lt.size()) > all || part == P.count) return;
     auto put = [&](DevBuf<RowBlock>& d, const std::vector<RowBlock>& h) {
         if (d.size() < h.size()) d.reset(h.size());  // a buffer only grows: graphs keep their pointer
         d.upload(h.data(), h.size(), P.stream);
@@ -898,7 +1254,7 @@ void set_phase_lists(Problem& P) {
     put(P.list_a, la);
     put(P.list_t, lt);
     P.list_na = static_cast<int>(la.size());
-    P.list_nt = static_cast<int>(lt.size());
+    P.list_nt = static_cast<int>(lt.size());  // 0: every instance of the phase is on chip
     P.list_level = level_index<M, V>();
     if (trace_enabled())
         std::fprintf(stderr, "[gb trace] phase lists: %d + %d of %d row blocks\n", P.list_na, P.list_nt,
@@ -918,10 +1274,12 @@ void run_phase(Problem& P, const gb_options* opt, double tol, int stall_exit, in
     long long checks_before = 0;
     if (!first)
         for (int k = 0; k < P.count; ++k) checks_before = std::max<long long>(checks_before, P.st_host[k].checks);
-    GB_CUDA(cudaMemcpyAsync(P.phase_flags.get(), P.phase_flags_host, sizeof(int) * P.count, cudaMemcpyHostToDevice,
-                            s));
+    P.phase_flags_host[P.count] = 0;
+    GB_CUDA(cudaMemcpyAsync(P.phase_flags.get(), P.phase_flags_host, sizeof(int) * (P.count + 1),
+                            cudaMemcpyHostToDevice, s));
     k_set_phase<<<div_up(P.count, kThreads), kThreads, 0, s>>>(P.count, P.st.get(), P.phase_flags.get(), tol,
                                                                stall_checks, stall_exit, first ? 1 : 0);
+    prepare_resident<M, V>(P);
     set_phase_lists<M, V>(P);
     PhaseListsOff lists_off{P};
     k_phase_in<V><<<gv, kThreads, 0, s>>>(P.n, P.m, P.icol(), P.irow(), P.st.get(), P.x64.get(), P.y64.get(),
@@ -957,6 +1315,8 @@ void run_phase(Problem& P, const gb_options* opt, double tol, int stall_exit, in
     k_phase_out<V><<<gv, kThreads, 0, s>>>(P.n, P.m, P.icol(), P.irow(), vs.x0.get(), vs.y0.get(), vs.sumx.get(),
                                           vs.sumy.get(), vs.xr.get(), vs.yr.get(), P.st.get(), P.x64.get(),
                                           P.y64.get(), P.xr64.get(), P.yr64.get());
+    GB_CUDA(cudaMemcpyAsync(P.phase_flags_host + P.count, P.phase_flags.get() + P.count, sizeof(int),
+                            cudaMemcpyDeviceToHost, s));
     sync_state(P);
     if (!host_loop_mode()) {
         long long checks_after = 0;
@@ -965,6 +1325,7 @@ void run_phase(Problem& P, const gb_options* opt, double tol, int stall_exit, in
     }
     P.launches += 1 + bodies * per_body;
     GB_CUDA(cudaGetLastError());
+    if (P.phase_flags_host[P.count]) throw Error(GB_ERR_CUDA, "an exchange between the CTAs of a cluster timed out");
 }
 
 // pdhg_evaluate<Bd> (pdhg_impl.hpp:202-230) of the carried FP64 state of every instance.
@@ -1240,6 +1601,7 @@ void rebuild_schedules(Problem& P, int w) {
     cudaStream_t s = P.stream;
     GB_CUDA(cudaStreamSynchronize(s));
     for (auto& g : P.graphs) g.reset();
+    for (ResPlan& r : P.res) r = ResPlan{};  // packed by these schedules' lanes per row
     DevSchedule& sa = w == 0 ? P.A.sched32 : P.A.sched;
     DevSchedule& st = w == 0 ? P.AT.sched32 : P.AT.sched;
     sa.upload(build_schedule(P.A.host_ptr.data(), P.row_off.data(), P.count, P.tune_block_nnz[w].data(),

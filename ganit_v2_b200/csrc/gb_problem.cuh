@@ -9,6 +9,7 @@
 
 #include "../../include/ganit_b200.h"
 #include "gb_pdhg.cuh"
+#include "gb_resident.cuh"
 #include "gb_setup.cuh"
 
 namespace gb {
@@ -132,8 +133,8 @@ struct Problem {
     VecSet<double> v64;
     DevBuf<SolveState> st;                // per instance
     SolveState* st_host = nullptr;        // pinned mirror (count entries)
-    DevBuf<int> phase_flags;              // per-instance flags uploaded for a phase
-    int* phase_flags_host = nullptr;      // pinned
+    DevBuf<int> phase_flags;              // per-instance flags uploaded for a phase; last entry: k_resident's error
+    int* phase_flags_host = nullptr;      // pinned (count + 1)
     DevBuf<double> partials;
     // Phase graphs: levels <f32,f32>, <f32,f64>, <f64,f64>, <bf16,f32>, then the
     // same four for phases that run on block lists.
@@ -141,10 +142,11 @@ struct Problem {
     DevBuf<double> w_start;               // per-instance primal weight of a warm start (<= 0: the default)
     // Row blocks of the current phase when only some instances of a batch take
     // part and their blocks are at most half of all: copies of those
-    // instances' RowBlocks, which the iteration kernels of level list_level
-    // run alone (list_level -1: none).
+    // instances' RowBlocks (without the on-chip ones, ResPlan), which the
+    // streaming kernels of level list_level run alone (list_level -1: none).
     DevBuf<RowBlock> list_a, list_t;
     int list_na = 0, list_nt = 0, list_level = -1;
+    ResPlan res[2];                       // instances iterated on chip: FP32 vectors, FP64 vectors
     double setup_seconds = 0.0;
     long long launches = 0;               // kernel launches of the last solve
     std::vector<InstanceResult> results;

@@ -1,0 +1,612 @@
+// On-chip PDHG iterations of small instances: one thread-block cluster keeps
+// an instance's scaled matrix, vectors and iterate in shared memory and runs
+// a whole check period (check_every iterations) in one launch.
+//
+// The streaming kernels (gb_pdhg.cuh) pay two dependent launches and a pass
+// over the matrix in L2 / HBM per iteration: 7-9 us an iteration on any LP
+// below ~1M nonzeros (launch latency), and the L1TEX wavefronts of random
+// global gathers on a large batch.  An instance of up to ~100K nonzeros fits
+// the shared memory of at most 16 SMs, so here
+//   * every CTA of the cluster owns a share of A^T's rows (columns of the LP)
+//     and of A's rows, with their matrix entries in shared memory;
+//   * every CTA holds a full copy of the two gathered vectors (xbar and y), so
+//     a gather is a shared-memory read.  After each half iteration a CTA sends
+//     its share to every other one with a bulk copy between shared memories,
+//     which counts its bytes on the receiver's mbarrier; the receiver starts
+//     its next half when all shares are in.  A share of iteration k + 1
+//     cannot overtake one of iteration k: it depends on the receiver's own
+//     share of the half in between, sent after its last read.
+//
+// Layout ("slices").  Rows are reduced by groups of G = 2^lg lanes, lane g of
+// a group adding entries g, g + G, ... of its row in order, then the groups'
+// shuffle tree -- for FP32 vectors exactly spmv_run's order with the row
+// block's own lg, so an FP32 iterate has the same bits on either path.  (FP64
+// kernels stream with the segmented order of spmv_run_seg; here lg comes from
+// the row's length alone, so an instance's result does not depend on what
+// shares its batch.)  A slice is 32 >> lg rows, one warp; rows are sorted by
+// their number of lane steps, so slices carry almost no padding, and a
+// slice's entries are stored step-major in pairs: for pair t, 32 words of two
+// 16-bit column positions and 32 pairs of values -- conflict-free reads
+// whatever the row lengths.  Columns and rows are renumbered by their place
+// in that order (owner-major), so an owner's entries are contiguous in the
+// gathered vectors.  Padding entries point at a slot that holds 0 with value
+// 0; a sum that started at +0 is unchanged by adding +0.
+#pragma once
+#include <algorithm>
+#include <array>
+#include <cstring>
+#include <vector>
+
+#include "gb_pdhg.cuh"
+
+namespace gb {
+
+constexpr int kResMaxSteps = 32;                       // lane steps of a row (kMaxLaneSum of a STREAM block)
+constexpr int kResBins = kResMaxSteps / 2 + 1;         // step pairs 0..16
+constexpr int kResMaxIndex = 65535;                    // positions are 16 bits wide
+constexpr size_t kResMaxSmem = 227 * 1024;             // shared memory of one CTA
+constexpr int kResMaxCluster = 16;
+constexpr int kResLaneSteps64 = 8;                     // FP64: lanes per row so that a lane adds at most this many
+
+// One CTA's share of an instance.
+struct ResCta {
+    int inst;
+    int slice0, ns_t, ns_a;   // its slices: ns_t of A^T, then ns_a of A
+    int pairs;                // step pairs stored (A^T's slices, then A's)
+    int own_t, own_a;         // columns / rows it owns
+    int pos_t0, pos_a0;       // their first positions in the instance (multiples of 4: 16-byte copies)
+    int n, m;                 // positions of the instance's columns / rows; entries n and m are the zero slots
+    int at_t0, at_a0;         // the instance's first entries of col_at / row_at
+    int pairs_t;              // A^T's step pairs, stored before A's
+    long long pair0;          // first step pair in the packed arrays
+};
+
+// A slice in shared memory: {first pair, pairs | lg << 8 | rows << 12, first own index, first position}.
+struct ResSlice {
+    int pair0, meta, own0, pos0;
+};
+static_assert(sizeof(ResSlice) == 16, "slices are read as one 16-byte word");
+
+// Launch class: instances with the same cluster size and shared-memory bucket.
+struct ResClass {
+    int cluster = 1, threads = 256;
+    int cta0 = 0, nctas = 0;
+    size_t smem = 0;
+};
+
+constexpr size_t kResBarBytes = 16;  // two mbarriers
+
+template <class V>
+__host__ __device__ inline size_t res_vec_bytes(int n, int m, int own_t, int own_a) {
+    auto r4 = [](int k) { return static_cast<size_t>((k + 3) & ~3); };
+    return kResBarBytes + sizeof(V) * (r4(n + 1) + r4(m + 1) + 5 * r4(own_t) + 3 * r4(own_a));
+}
+template <class M, class V>
+__host__ __device__ inline size_t res_smem_bytes(int slices, int pairs, int n, int m, int own_t, int own_a) {
+    return 16 * static_cast<size_t>(slices) + static_cast<size_t>(pairs) * (128 + 64 * sizeof(M)) +
+           res_vec_bytes<V>(n, m, own_t, own_a);
+}
+
+// ---------------------------------------------------------------- device
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Barrier over the cluster's threads; what they wrote to any of its shared
+// memories before it is visible after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(r)
+                 : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
+    return r;
+}
+
+// mbarriers of one arrival (the CTA's own) plus the bytes announced with it.
+__device__ __forceinline__ void mbar_init(unsigned long long* b) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b)))
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init_visible() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mbar_expect(unsigned long long* b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(b))),
+                 "r"(bytes)
+                 : "memory");
+}
+// Waits for the phase of the given parity; false after kResWaitTries tries
+// (each suspends the thread for a while), which only a broken copy can cause.
+constexpr int kResWaitTries = 1 << 18;
+__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
+    const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(b));
+    for (int k = 0; k < kResWaitTries; ++k) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// Own shared memory -> the same place of CTA `rank`, counted on its mbarrier.
+__device__ __forceinline__ void copy_to_peer(const void* p, unsigned bytes, unsigned long long* bar, int rank) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     cluster_addr(p, rank)),
+                 "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(bytes), "r"(cluster_addr(bar, rank))
+                 : "memory");
+}
+// Shared-memory writes of this thread, before a bulk copy reads them.
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Two matrix values of a lane's step pair.
+__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    a = v.x; b = v.y;
+}
+__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    a = v.x; b = v.y;
+}
+__device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, __nv_bfloat16& a, __nv_bfloat16& b) {
+    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(p);
+    a = v.x; b = v.y;
+}
+
+// Row sums of a slice: a lane's part over its steps, then the group's tree
+// (the sum lands in each group's first lane).
+template <class M, class V>
+__device__ __forceinline__ V slice_sum(int pair0, int np, int lg, const unsigned* idx, const M* val, const V* g,
+                                       int lane) {
+    const unsigned* ip = idx + pair0 * 32 + lane;
+    const M* vp = val + pair0 * 64 + 2 * lane;
+    V acc = V(0);
+#pragma unroll 4
+    for (int t = 0; t < np; ++t) {
+        const unsigned j = ip[32 * t];
+        M a, b;
+        ld_pair(vp + 64 * t, a, b);
+        acc += static_cast<V>(a) * g[j & 0xffffu];
+        acc += static_cast<V>(b) * g[j >> 16];
+    }
+    if (lg > 4) acc += __shfl_down_sync(0xffffffffu, acc, 16);
+    if (lg > 3) acc += __shfl_down_sync(0xffffffffu, acc, 8);
+    if (lg > 2) acc += __shfl_down_sync(0xffffffffu, acc, 4);
+    if (lg > 1) acc += __shfl_down_sync(0xffffffffu, acc, 2);
+    if (lg > 0) acc += __shfl_down_sync(0xffffffffu, acc, 1);
+    return acc;
+}
+
+template <class M, class V>
+struct ResArgs {
+    const ResCta* cta;        // records of this class
+    const ResSlice* slices;
+    const unsigned* idx;      // packed position pairs
+    const M* val;             // packed value pairs
+    const int* col_at;        // position -> column (global), per instance from its first column
+    const int* row_at;
+    const V* x0; const V* y0; // iterate in
+    V* x; V* y;               // iterate out
+    V* sumx; V* sumy;
+    const V* c; const V* l; const V* u; const V* lo; const V* hi;
+    SolveState* st;
+    int* error;               // set when a wait ran out
+    int iters, cluster;
+};
+
+template <class M, class V, int T>
+__global__ void __launch_bounds__(T) k_resident(const __grid_constant__ ResArgs<M, V> a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const ResCta r = a.cta[blockIdx.x];
+    const SolveState& s = a.st[r.inst];
+    if (s.active == 0) return;  // the same for every CTA of the cluster
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int W = T / 32;
+    auto r4 = [](int k) { return (k + 3) & ~3; };
+    // the gathered vectors first: their place is the same in every CTA of the cluster
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);  // [0] xbar, [1] y
+    V* xs = reinterpret_cast<V*>(smem + kResBarBytes);  // xbar by position, all columns
+    V* ys = xs + r4(r.n + 1);                          // y by position, all rows
+    ResSlice* sl = reinterpret_cast<ResSlice*>(ys + r4(r.m + 1));
+    unsigned* idx = reinterpret_cast<unsigned*>(sl + r.ns_t + r.ns_a);
+    M* val = reinterpret_cast<M*>(idx + 32 * r.pairs);
+    V* ox = reinterpret_cast<V*>(val + 64 * r.pairs);
+    V* oc = ox + r4(r.own_t);
+    V* ol = oc + r4(r.own_t);
+    V* ou = ol + r4(r.own_t);
+    V* osx = ou + r4(r.own_t);
+    V* olo = osx + r4(r.own_t);
+    V* ohi = olo + r4(r.own_a);
+    V* osy = ohi + r4(r.own_a);
+    // matrix share and slice table: asynchronous copies; vectors meanwhile
+    for (int k = tid; k < r.ns_t + r.ns_a; k += T) cp_async16(sl + k, a.slices + r.slice0 + k);
+    for (int k = tid; k < 8 * r.pairs; k += T) cp_async16(idx + 4 * k, a.idx + 32 * r.pair0 + 4 * k);
+    constexpr int kPer16 = 16 / static_cast<int>(sizeof(M));
+    for (int k = tid; k < 64 / kPer16 * r.pairs; k += T) cp_async16(val + kPer16 * k, a.val + 64 * r.pair0 + kPer16 * k);
+    for (int k = tid; k < r.own_t; k += T) {
+        const int j = a.col_at[r.at_t0 + r.pos_t0 + k];
+        ox[k] = a.x0[j];
+        oc[k] = a.c[j];
+        ol[k] = a.l[j];
+        ou[k] = a.u[j];
+        osx[k] = a.sumx[j];
+    }
+    for (int k = tid; k < r.own_a; k += T) {
+        const int i = a.row_at[r.at_a0 + r.pos_a0 + k];
+        olo[k] = a.lo[i];
+        ohi[k] = a.hi[i];
+        osy[k] = a.sumy[i];
+    }
+    for (int k = tid; k < r.m; k += T) {
+        const int i = a.row_at[r.at_a0 + k];
+        ys[k] = i >= 0 ? a.y0[i] : V(0);  // -1: between two shares
+    }
+    if (tid == 0) {
+        xs[r.n] = V(0);
+        ys[r.m] = V(0);
+        mbar_init(bar);
+        mbar_init(bar + 1);
+        mbar_init_visible();
+    }
+    const V tau = static_cast<V>(s.tau), sigma = static_cast<V>(s.sigma);
+    cp_async_wait_all();
+    const int rank = static_cast<int>(blockIdx.x) % a.cluster;
+    const unsigned bytes_x = sizeof(V) * r4(r.own_t), bytes_y = sizeof(V) * r4(r.own_a);
+    bool lost = false;
+    // End of a half: this CTA's share `p` of a gathered vector goes to every
+    // other CTA, and theirs are awaited (total: the vector's bytes).
+    auto exchange = [&](const V* p, unsigned bytes, unsigned total, int b, int it) {
+        if (a.cluster == 1) {
+            __syncthreads();
+            return;
+        }
+        fence_async_proxy();
+        __syncthreads();
+        if (warp == 0) {
+            if (lane == 0) mbar_expect(bar + b, total - bytes);
+            if (lane < a.cluster && lane != rank && bytes) copy_to_peer(p, bytes, bar + b, lane);
+        }
+        if (!lost) lost = !mbar_wait(bar + b, it & 1);
+    };
+    if (a.cluster > 1) cluster_sync();  // every CTA has started and holds its share
+    else __syncthreads();
+    for (int it = 0; it < a.iters; ++it) {
+        for (int q = warp; q < r.ns_t; q += W) {  // primal half (PrimalEpi)
+            const ResSlice e = sl[q];
+            const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
+            const int k = e.own0 + grp;
+            const V xk = ox[k], ck = oc[k], lk = ol[k], uk = ou[k], sk = osx[k];
+            const V t = slice_sum<M, V>(e.pair0, np, lg, idx, val, ys, lane);
+            const V g = ck - t + V(0);
+            V v = xk - tau * g;
+            v = (v < lk) ? lk : v;
+            v = (uk < v) ? uk : v;
+            if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < nr) {
+                ox[k] = v;
+                osx[k] = sk + v;
+                xs[e.pos0 + grp] = V(2) * v - xk;
+            }
+        }
+        exchange(xs + r.pos_t0, bytes_x, sizeof(V) * r.n, 0, it);
+        for (int q = r.ns_t + warp; q < r.ns_t + r.ns_a; q += W) {  // dual half (DualEpi)
+            const ResSlice e = sl[q];
+            const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
+            const int k = e.own0 + grp;
+            const V yk = ys[e.pos0 + grp], sk = osy[k], lk = sigma * olo[k], hk = sigma * ohi[k];
+            const V t = slice_sum<M, V>(e.pair0, np, lg, idx, val, xs, lane);
+            const V qv = yk - sigma * t;
+            V w = -qv;
+            w = (w < lk) ? lk : w;
+            w = (hk < w) ? hk : w;
+            const V v = qv + w;
+            if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < nr) {
+                osy[k] = sk + v;
+                ys[e.pos0 + grp] = v;
+            }
+        }
+        exchange(ys + r.pos_a0, bytes_y, sizeof(V) * r.m, 1, it);
+    }
+    if (lost) {  // the solve stops at the coming check and reports the error
+        atomicExch(a.error, 1);
+        a.st[r.inst].max_iter = 0;
+    }
+    for (int k = tid; k < r.own_t; k += T) {
+        const int j = a.col_at[r.at_t0 + r.pos_t0 + k];
+        a.x[j] = ox[k];
+        a.sumx[j] = osx[k];
+    }
+    for (int k = tid; k < r.own_a; k += T) {
+        const int i = a.row_at[r.at_a0 + r.pos_a0 + k];
+        a.y[i] = ys[r.pos_a0 + k];
+        a.sumy[i] = osy[k];
+    }
+    if (a.cluster > 1) cluster_sync();  // no CTA leaves while a copy may still read its share
+}
+
+// ---------------------------------------------------------------- packing (device, once per plan)
+// Lanes per row: lg of the STREAM block that holds it (FP32 vectors).
+static __global__ void k_res_row_lg(int nb, const RowBlock* __restrict__ blocks, unsigned char* __restrict__ lg) {
+    const RowBlock b = blocks[blockIdx.x];
+    for (int r = b.r0 + threadIdx.x; r < b.r1; r += blockDim.x) lg[r] = static_cast<unsigned char>(b.lg);
+}
+__host__ __device__ inline int res_lg64(int len) {
+    int lg = 0;
+    while (lg < 5 && (kResLaneSteps64 << lg) < len) ++lg;
+    return lg;
+}
+
+// One side (A^T's or A's rows) of one resident instance, for the packing kernels.
+struct ResSide {
+    int row0, row1;                        // global rows of the side's matrix
+    int at0;                               // first entry of the position -> row list
+    int slice0[6];                         // first entry of the side's slices of each lg in the slice list
+    int rank0[6][kResBins];                // rank of the first row of (lg, pairs) among the rows of lg
+};
+struct ResSliceAt {                        // slice list entry: where the slice lives
+    long long pair0;                       // global first pair
+    int meta, pos0;
+};
+
+// One warp per side walks its rows in order and gives every row its slot
+// (slice list entry * 32 + group) and its position.
+static __global__ void k_res_rank(const ResSide* __restrict__ sides, const int* __restrict__ ptr,
+                                  const unsigned char* __restrict__ lg_of, const ResSliceAt* __restrict__ slices,
+                                  int* __restrict__ slot, unsigned short* __restrict__ pos, int* __restrict__ at) {
+    __shared__ int next[6 * kResBins];
+    const ResSide& sd = sides[blockIdx.x];
+    const int lane = threadIdx.x;
+    for (int k = lane; k < 6 * kResBins; k += 32) next[k] = sd.rank0[k / kResBins][k % kResBins];
+    __syncwarp();
+    for (int r0 = sd.row0; r0 < sd.row1; r0 += 32) {
+        const int r = r0 + lane;
+        int bin = -1, lg = 0;
+        if (r < sd.row1) {
+            const int len = ptr[r + 1] - ptr[r];
+            lg = lg_of ? lg_of[r] : res_lg64(len);
+            const int steps = (len + (1 << lg) - 1) >> lg;
+            bin = lg * kResBins + ((steps + 1) >> 1);
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, bin);
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        int base = 0;
+        if (bin >= 0) base = next[bin];
+        __syncwarp();
+        if (bin >= 0 && rank == 0) next[bin] = base + __popc(peers);
+        __syncwarp();
+        if (bin >= 0) {
+            const int k = base + rank, rows = 32 >> lg;
+            const int e = sd.slice0[lg] + k / rows, grp = k % rows;
+            const int p = slices[e].pos0 + grp;
+            slot[r] = e * 32 + grp;
+            pos[r] = static_cast<unsigned short>(p);
+            at[sd.at0 + p] = r;
+        }
+    }
+}
+
+// Every packed pair starts as padding: the zero slot's position, value 0.
+static __global__ void k_res_fill(const ResCta* __restrict__ cta, unsigned* __restrict__ idx) {
+    const ResCta r = cta[blockIdx.x];
+    // A^T's pairs gather y (zero slot m), A's gather xbar (zero slot n)
+    const unsigned zt = static_cast<unsigned>(r.m) * 0x10001u, za = static_cast<unsigned>(r.n) * 0x10001u;
+    for (int k = threadIdx.x; k < 32 * r.pairs; k += blockDim.x) idx[32 * r.pair0 + k] = k < 32 * r.pairs_t ? zt : za;
+}
+
+// Entries of the rows of one side: positions (from the other side's
+// numbering) and, through k_res_values, values.
+static __global__ void k_res_entries(int rows, const int* __restrict__ ptr, const int* __restrict__ col,
+                                     const int* __restrict__ slot, const ResSliceAt* __restrict__ slices,
+                                     const unsigned short* __restrict__ pos_other, unsigned short* __restrict__ idx) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+        const int sr = slot[r];
+        if (sr < 0) continue;  // the row's instance is not resident
+        const ResSliceAt e = slices[sr >> 5];
+        const int lg = (e.meta >> 8) & 0xf, G = 1 << lg, p0 = ptr[r], len = ptr[r + 1] - p0;
+        for (int k = 0; k < len; ++k) {
+            const int t = k >> lg, lane = ((sr & 31) << lg) + (k & (G - 1));
+            idx[(e.pair0 + (t >> 1)) * 64 + 2 * lane + (t & 1)] = pos_other[col[p0 + k]];
+        }
+    }
+}
+template <class M, class S>
+__global__ void k_res_values(int rows, const int* __restrict__ ptr, const S* __restrict__ val,
+                             const int* __restrict__ slot, const ResSliceAt* __restrict__ slices, M* __restrict__ out) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+        const int sr = slot[r];
+        if (sr < 0) continue;
+        const ResSliceAt e = slices[sr >> 5];
+        const int lg = (e.meta >> 8) & 0xf, G = 1 << lg, p0 = ptr[r], len = ptr[r + 1] - p0;
+        for (int k = 0; k < len; ++k) {
+            const int t = k >> lg, lane = ((sr & 31) << lg) + (k & (G - 1));
+            out[(e.pair0 + (t >> 1)) * 64 + 2 * lane + (t & 1)] = static_cast<M>(val[p0 + k]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- host: who is resident, and where
+// Row counts of one side by (lg, step pairs); false: a row it cannot hold.
+struct ResHist {
+    int h[6][kResBins] = {};
+    long long pairs = 0;  // over slices
+    int slices = 0;
+    // slices of each lg: pairs of the k-th (rows in order of falling pairs)
+    template <class F>
+    void each_slice(F&& f) const {
+        for (int lg = 0; lg < 6; ++lg) {
+            const int rows = 32 >> lg;
+            int left = 0, fill = 0, top = 0;
+            for (int b = kResBins - 1; b >= 0; --b) left += h[lg][b];
+            for (int b = kResBins - 1; b >= 0 && left > 0; --b) {
+                int c = h[lg][b];
+                while (c > 0) {
+                    if (fill == 0) top = b;
+                    const int take = std::min(c, rows - fill);
+                    fill += take;
+                    c -= take;
+                    left -= take;
+                    if (fill == rows || left == 0) {
+                        f(lg, top, fill);
+                        fill = 0;
+                    }
+                }
+            }
+        }
+    }
+    void count() {
+        pairs = 0;
+        slices = 0;
+        each_slice([&](int, int np, int) {
+            pairs += np;
+            ++slices;
+        });
+    }
+};
+inline bool res_hist_rows(const int* ptr, int r0, int r1, int lg_fixed, ResHist& H) {
+    for (int r = r0; r < r1; ++r) {
+        const int len = ptr[r + 1] - ptr[r];
+        const int lg = lg_fixed >= 0 ? lg_fixed : res_lg64(len);
+        const int steps = (len + (1 << lg) - 1) >> lg;
+        if (steps > kResMaxSteps) return false;
+        ++H.h[lg][(steps + 1) >> 1];
+    }
+    return true;
+}
+
+// Slices of both sides of an instance dealt to C CTAs: by falling pairs, back
+// and forth over the CTAs, so the shares differ by about one slice.
+struct ResDeal {
+    struct Item {
+        int lg, pairs, rows, cta, ord;  // ord: place among the CTA's slices of its side
+        int own0, pos0, pair0;
+    };
+    std::vector<Item> side[2];      // A^T, A; in slice list order (lg-major)
+    std::vector<ResCta> cta;
+    size_t smem(size_t sm, size_t sv) const {
+        size_t top = 0;
+        for (const ResCta& c : cta) {
+            const size_t b = sm == 8 ? res_smem_bytes<double, double>(c.ns_t + c.ns_a, c.pairs, c.n, c.m, c.own_t, c.own_a)
+                             : sv == 8 ? res_smem_bytes<float, double>(c.ns_t + c.ns_a, c.pairs, c.n, c.m, c.own_t, c.own_a)
+                                       : res_smem_bytes<float, float>(c.ns_t + c.ns_a, c.pairs, c.n, c.m, c.own_t, c.own_a);
+            top = std::max(top, b);
+        }
+        return top;
+    }
+};
+inline void res_deal(const std::array<ResHist, 2>& H, int C, ResDeal& D) {
+    D.cta.assign(C, ResCta{});
+    for (int sd = 0; sd < 2; ++sd) {
+        auto& it = D.side[sd];
+        it.clear();
+        it.reserve(H[sd].slices);
+        H[sd].each_slice([&](int lg, int np, int rows) { it.push_back({lg, np, rows, 0, 0, 0, 0, 0}); });
+        std::vector<int> order(it.size());
+        std::array<int, kResBins + 1> start{};
+        for (const auto& e : it) ++start[kResBins - 1 - e.pairs + 1];
+        for (int b = 0; b < kResBins; ++b) start[b + 1] += start[b];
+        for (size_t k = 0; k < it.size(); ++k) order[start[kResBins - 1 - it[k].pairs]++] = static_cast<int>(k);
+        std::vector<int> own(C, 0);
+        for (size_t q = 0; q < order.size(); ++q) {
+            const int lap = static_cast<int>(q / C), at = static_cast<int>(q % C);
+            const int c = (lap & 1) ? C - 1 - at : at;
+            auto& e = it[order[q]];
+            ResCta& k = D.cta[c];
+            e.cta = c;
+            e.ord = sd == 0 ? k.ns_t++ : k.ns_a++;
+            e.pair0 = k.pairs;
+            e.own0 = own[c];
+            own[c] += e.rows;
+            k.pairs += e.pairs;
+        }
+        int pos = 0;
+        for (int c = 0; c < C; ++c) {
+            (sd == 0 ? D.cta[c].own_t : D.cta[c].own_a) = own[c];
+            (sd == 0 ? D.cta[c].pos_t0 : D.cta[c].pos_a0) = pos;
+            pos += (own[c] + 3) & ~3;
+            if (sd == 0) D.cta[c].pairs_t = D.cta[c].pairs;
+        }
+        for (ResCta& k : D.cta) (sd == 0 ? k.n : k.m) = pos;
+        for (auto& e : it) e.pos0 = (sd == 0 ? D.cta[e.cta].pos_t0 : D.cta[e.cta].pos_a0) + e.own0;
+    }
+}
+
+// Device tables of the resident instances, filled instance by instance.
+struct ResTables {
+    std::vector<ResCta> cta;
+    std::vector<ResSlice> slices;
+    std::vector<ResSliceAt> at;
+    std::vector<ResSide> sides[2];  // A^T, A
+    long long pairs = 0;
+    int positions[2] = {0, 0};      // entries of col_at, row_at
+    void add(int inst, const std::array<ResHist, 2>& H, const ResDeal& D, int col0, int col1, int row0, int row1) {
+        const size_t c0 = cta.size();
+        for (ResCta k : D.cta) {
+            k.inst = inst;
+            k.at_t0 = positions[0];
+            k.at_a0 = positions[1];
+            k.pair0 = pairs;
+            k.slice0 = static_cast<int>(slices.size());
+            pairs += k.pairs;
+            slices.resize(slices.size() + k.ns_t + k.ns_a);
+            cta.push_back(k);
+        }
+        for (int sd = 0; sd < 2; ++sd) {
+            ResSide s{};
+            s.row0 = sd == 0 ? col0 : row0;
+            s.row1 = sd == 0 ? col1 : row1;
+            s.at0 = positions[sd];
+            for (int lg = 0; lg < 6; ++lg) {
+                int run = 0;
+                for (int b = kResBins - 1; b >= 0; --b) {
+                    s.rank0[lg][b] = run;
+                    run += H[sd].h[lg][b];
+                }
+                s.slice0[lg] = -1;
+            }
+            for (const auto& e : D.side[sd]) {
+                if (s.slice0[e.lg] < 0) s.slice0[e.lg] = static_cast<int>(at.size());
+                const ResCta& k = cta[c0 + e.cta];
+                const int meta = e.pairs | e.lg << 8 | e.rows << 12;
+                at.push_back({k.pair0 + e.pair0, meta, e.pos0});
+                slices[k.slice0 + (sd == 0 ? 0 : k.ns_t) + e.ord] = {e.pair0, meta, e.own0, e.pos0};
+            }
+            sides[sd].push_back(s);
+        }
+        positions[0] += D.cta[0].n;
+        positions[1] += D.cta[0].m;
+    }
+};
+
+// The resident instances of a problem for one vector precision.
+struct ResPlan {
+    bool built = false;
+    std::vector<char> resident;             // per instance
+    std::vector<ResClass> classes;
+    DevBuf<ResCta> cta;
+    DevBuf<ResSlice> slices;
+    DevBuf<unsigned> idx;
+    DevBuf<float> val32;
+    DevBuf<double> val64;
+    DevBuf<__nv_bfloat16> valbf;
+    DevBuf<int> col_at, row_at, slot_t, slot_a;
+    DevBuf<ResSliceAt> at;
+    DevBuf<ResSide> sides_t, sides_a;       // packing scratch, freed with the plan
+    DevBuf<unsigned short> pos_t, pos_a;
+    DevBuf<unsigned char> lg_t, lg_a;
+    long long pairs = 0;
+    // Row blocks of the other instances, which the streaming kernels run
+    // (nothing: every instance is resident).
+    DevBuf<RowBlock> list_a, list_t;
+    int list_na = 0, list_nt = 0;
+    bool any() const { return !classes.empty(); }
+};
+
+}  // namespace gb
