@@ -257,6 +257,9 @@ void init_kernel_attrs() {
         init_resident_attrs<__nv_bfloat16, float>();
         init_resident_attrs<float, double>();
         init_resident_attrs<double, double>();
+        set_smem(k_qp_chip<float, float>, kQpSmem);
+        set_smem(k_qp_chip<float, double>, kQpSmem);
+        set_smem(k_qp_chip<double, double>, kQpSmem);
     });
 }
 
@@ -954,11 +957,95 @@ void ensure_resident(Problem& P) {
                          c.nctas, c.cluster, c.threads, c.smem);
 }
 
+// Whether level <M, V> of a QP runs k_qp_chip: a diagonal-plus-low-rank
+// Hessian, at most kQpMaxRows rows with as many entries a column, one CTA per
+// SM with a column per thread, and F on chip (qp_smem_rows: all of it in
+// shared memory, in FP64 the rest in registers; beyond, the streaming kernels
+// read it from L2 with eight CTAs per SM).
+template <class M, class V>
+bool qp_on_chip(const Problem& P) {
+    int rows_per = 0;
+    if (!P.dplr || P.m > kQpMaxRows || P.sms < kQpGrid || !resident_enabled()) return false;
+    if (qp_smem_rows<V>(P.n, P.qk, &rows_per) == 0) return false;
+    if (P.A.template sched_for<M>().nb + P.m > kQpMaxSlots) return false;
+    for (int j = 0; j < P.n; ++j)
+        if (P.AT.host_ptr[j + 1] - P.AT.host_ptr[j] > kQpMaxRows) return false;
+    return true;
+}
+
+template <class M, class V>
+void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
+    const bool odd = (ce & 1) != 0;
+    QpArgs<M, V> a{};
+    a.n = P.n;
+    a.m = P.m;
+    a.k = P.qk;
+    a.iters = ce;
+    a.smem_rows = qp_smem_rows<V>(P.n, P.qk, &a.rows_per);
+    a.F = vs.F.get();
+    a.D = vs.D.get();
+    a.c = vs.c.get();
+    a.l = vs.l.get();
+    a.u = vs.u.get();
+    a.lo = vs.lo.get();
+    a.hi = vs.hi.get();
+    a.at_ptr = P.AT.ptr.get();
+    a.at_idx = P.AT.idx.get();
+    a.at_val = P.AT.val<M>();
+    a.at_lg = sizeof(V) == 4 ? P.qp_at_lg.get() : nullptr;
+    a.A = P.A.view<M>();
+    a.slots = P.qp_slots.get();
+    const std::vector<RowBlock>& blocks = P.A.template sched_for<M>().host_blocks;
+    for (int b = 0; b < a.A.nb; ++b)
+        for (int r = blocks[b].r0; r < blocks[b].r1; ++r) {
+            if (blocks[b].kind == kStream) a.slot0[r] = a.A.nb + r;
+            else if (a.nslots[r] == 0) a.slot0[r] = b;
+            ++a.nslots[r];
+        }
+    a.total_slots = a.A.nb + P.m;
+    a.x0 = vs.x0.get();
+    a.y0 = vs.y0.get();
+    a.x = odd ? vs.x1.get() : vs.x0.get();
+    a.y = odd ? vs.y1.get() : vs.y0.get();
+    a.xbar = vs.xbar.get();
+    a.sumx = vs.sumx.get();
+    a.sumy = vs.sumy.get();
+    a.part = P.partials.get();
+    a.t = P.ftx.get();
+    a.st = a.st_rw = P.st.get();
+    a.sync = P.qp_sync.get();
+    a.error = P.phase_flags.get() + P.count;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(kQpGrid);
+    cfg.blockDim = dim3(kQpThreads);
+    cfg.dynamicSmemBytes = kQpSmem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeCooperative;  // its CTAs wait for one another
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GB_CUDA(cudaLaunchKernelEx(&cfg, k_qp_chip<M, V>, a));
+}
+
 // What a body of level <M, V> needs on chip; before its graph is captured.
 template <class M, class V>
 void prepare_resident(Problem& P) {
     ensure_resident<V>(P);
     ensure_resident_values<M, V>(P);
+    if (P.dplr && !P.qp_sync.get()) {
+        P.qp_sync.reset(2);
+        GB_CUDA(cudaMemsetAsync(P.qp_sync.get(), 0, 2 * sizeof(unsigned), P.stream));
+        P.qp_slots.reset(kQpMaxSlots);
+        GB_CUDA(cudaMemsetAsync(P.qp_slots.get(), 0, kQpMaxSlots * sizeof(double), P.stream));
+    }
+    if (P.dplr && sizeof(V) == 4 && !P.qp_at_lg.get() && qp_on_chip<float, V>(P)) {
+        const DevSchedule& st = P.AT.template sched_for<V>();
+        P.qp_at_lg.reset(P.n);
+        GB_CUDA(cudaMemsetAsync(P.qp_at_lg.get(), 0, P.n, P.stream));
+        k_res_row_lg<<<st.nb, kThreads, 0, P.stream>>>(st.nb, st.blocks.get(), P.qp_at_lg.get());
+        GB_CUDA(cudaGetLastError());
+    }
 }
 
 // One PDHG iteration (k-th inside the body) on buffers selected by parity.
@@ -1049,7 +1136,14 @@ long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cuda
         launch_resident<M, V>(P, vs, c, ce, s);
         ++nl;
     }
-    if (sb.na != 0) {
+    bool on_chip = false;
+    if constexpr (!std::is_same<M, __nv_bfloat16>::value)  // the BF16 level takes LPs only
+        if (qp_on_chip<M, V>(P)) {
+            launch_qp_chip<M, V>(P, vs, ce, s);
+            on_chip = true;
+            ++nl;
+        }
+    if (sb.na != 0 && !on_chip) {
         br.next();
         for (int k = 0; k < ce; ++k) launch_iteration<M, V>(P, vs, k, s, nl, nullptr, sb);
     }
@@ -1602,6 +1696,7 @@ void rebuild_schedules(Problem& P, int w) {
     GB_CUDA(cudaStreamSynchronize(s));
     for (auto& g : P.graphs) g.reset();
     for (ResPlan& r : P.res) r = ResPlan{};  // packed by these schedules' lanes per row
+    P.qp_at_lg.release();
     DevSchedule& sa = w == 0 ? P.A.sched32 : P.A.sched;
     DevSchedule& st = w == 0 ? P.AT.sched32 : P.AT.sched;
     sa.upload(build_schedule(P.A.host_ptr.data(), P.row_off.data(), P.count, P.tune_block_nnz[w].data(),

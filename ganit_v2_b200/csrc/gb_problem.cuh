@@ -9,6 +9,7 @@
 
 #include "../../include/ganit_b200.h"
 #include "gb_pdhg.cuh"
+#include "gb_qp_chip.cuh"
 #include "gb_resident.cuh"
 #include "gb_setup.cuh"
 
@@ -146,6 +147,9 @@ struct Problem {
     // streaming kernels of level list_level run alone (list_level -1: none).
     DevBuf<RowBlock> list_a, list_t;
     int list_na = 0, list_nt = 0, list_level = -1;
+    DevBuf<unsigned char> qp_at_lg;       // k_qp_chip: log2 lanes per row of A^T (FP32)
+    DevBuf<unsigned> qp_sync;             // k_qp_chip's {arrivals, exits}
+    DevBuf<double> qp_slots;              // and its row sums
     ResPlan res[2];                       // instances iterated on chip: FP32 vectors, FP64 vectors
     double setup_seconds = 0.0;
     long long launches = 0;               // kernel launches of the last solve
