@@ -332,6 +332,35 @@ __device__ __forceinline__ void mr_cta_sum(double (&v)[1], double* red) {
     __syncthreads();
 }
 
+// The scalar part of a step: Givens rotations, estimate and stopping test of
+// state `s` from alpha and beta^2 of the new Lanczos vector; bc = {beta, phi,
+// 1 / gamma, old epsilon, delta, 1 / beta} for the vector updates.
+__device__ __forceinline__ void mr_scalars(MrState& s, double alpha, double bn2, double* bc, int* done) {
+    const double bn = sqrt(bn2);
+    const double oldeps = s.epsln;
+    const double delta = s.cs * s.dbar + s.sn * alpha;
+    const double gbar = s.sn * s.dbar - s.cs * alpha;
+    s.epsln = s.sn * bn;
+    s.dbar = -s.cs * bn;
+    double gamma = sqrt(gbar * gbar + bn * bn);
+    if (!(gamma > 1e-300)) gamma = 1e-300;
+    s.cs = gbar / gamma;
+    s.sn = bn / gamma;
+    const double phi = s.cs * s.phibar;
+    s.phibar = s.sn * s.phibar;
+    s.beta = bn;
+    s.it += 1;
+    s.converged = (s.phibar <= s.tol * s.beta1) || !(bn > 1e-300);
+    s.done = s.converged || s.it >= s.max_it || !isfinite(s.phibar);
+    bc[0] = bn;
+    bc[1] = phi;
+    bc[2] = 1.0 / gamma;
+    bc[3] = oldeps;
+    bc[4] = delta;
+    bc[5] = bn > 1e-300 ? 1.0 / bn : 0.0;
+    *done = s.done;
+}
+
 template <int NT>
 __device__ __forceinline__ void mr_update_step(const MrVecs& a, int k, MrState* sp, double* red, double* bc) {
     const int c0 = a.col_off[k], c1 = a.col_off[k + 1], r0 = a.row_off[k], r1 = a.row_off[k + 1];
@@ -356,28 +385,9 @@ __device__ __forceinline__ void mr_update_step(const MrVecs& a, int k, MrState* 
     mr_cta_sum<NT>(v, red);
     if (threadIdx.x == 0) {
         MrState s = *sp;
-        const double bn = sqrt(v[0]);
-        const double oldeps = s.epsln;
-        const double delta = s.cs * s.dbar + s.sn * alpha;
-        const double gbar = s.sn * s.dbar - s.cs * alpha;
-        s.epsln = s.sn * bn;
-        s.dbar = -s.cs * bn;
-        double gamma = sqrt(gbar * gbar + bn * bn);
-        if (!(gamma > 1e-300)) gamma = 1e-300;
-        s.cs = gbar / gamma;
-        s.sn = bn / gamma;
-        const double phi = s.cs * s.phibar;
-        s.phibar = s.sn * s.phibar;
-        s.beta = bn;
-        s.it += 1;
-        s.converged = (s.phibar <= s.tol * s.beta1) || !(bn > 1e-300);
-        s.done = s.converged || s.it >= s.max_it || !isfinite(s.phibar);
+        int done = 0;
+        mr_scalars(s, alpha, v[0], bc, &done);
         *sp = s;
-        bc[1] = phi;
-        bc[2] = 1.0 / gamma;
-        bc[3] = oldeps;
-        bc[4] = delta;
-        bc[5] = bn > 1e-300 ? 1.0 / bn : 0.0;
     }
     __syncthreads();
     const double phi = bc[1], ig = bc[2], oldeps = bc[3], delta = bc[4], ib = bc[5];
@@ -454,6 +464,170 @@ __global__ void __launch_bounds__(kMrSolveThreads) k_mr_solve(const __grid_const
         mr_update_step<kMrSolveThreads>(a.v, k, sp, red, bc);
         __syncthreads();  // v and the state are written before the next step reads them
     }
+}
+
+// The same solve with the system on chip, for instances of at most
+// R * kMrSolveThreads free columns and as many dual-active rows whose B and
+// B^T fit in shared memory: a thread owns R entries of each part of every
+// vector in registers and forms p = K v for them (both lanes' sums of mr_rows,
+// then their sum), so a step reads shared memory alone and the sums keep
+// k_mr_solve's order and bits.  B and B^T lie entry-major (entry e of row i at
+// e * stride + i) with 16-bit positions: conflict-free but for the gathers.
+// k_mr_solve spent 9 us a step (48 systems of ~450 + 450, 4,000 nonzeros) on
+// chains of L2 reads: p, the vectors and B live in global memory there.
+// Bound now by the gathers' shared-memory wavefronts and the four barriers.
+// Differentiable layer on those 48 LPs, forward + backward: 66 -> 47 ms.
+struct MrChipShape {
+    int stride_d, stride_f;  // rows of B / B^T per entry layer (multiples of 32)
+    int len_d, len_f;        // entry layers
+    __host__ __device__ size_t bytes() const {
+        const size_t cells = static_cast<size_t>(stride_d) * len_d + static_cast<size_t>(stride_f) * len_f;
+        return 8 * (cells + stride_d + stride_f) + 2 * ((cells + 7) & ~size_t(7));
+    }
+};
+constexpr size_t kMrChipSmem = 226 * 1024;
+
+template <int R>
+__global__ void __launch_bounds__(kMrSolveThreads) k_mr_solve_chip(const __grid_constant__ MrOpArgs a,
+                                                                   const MrChipShape sh) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NT = kMrSolveThreads, NW = NT / 32;
+    __shared__ double red[NW], red2[NW], bc[6];
+    __shared__ int done;
+    const int k = blockIdx.x, tid = threadIdx.x;
+    MrState* sp = a.v.st + k;
+    if (sp->done) return;
+    const int f0 = a.v.col_off[k], nf = a.v.col_off[k + 1] - f0, d0 = a.v.row_off[k], nd = a.v.row_off[k + 1] - d0;
+    double* vd = reinterpret_cast<double*>(smem);  // values of B, then of B^T
+    double* vf = vd + static_cast<size_t>(sh.stride_d) * sh.len_d;
+    double* xs = vf + static_cast<size_t>(sh.stride_f) * sh.len_f;  // v by position
+    double* ys = xs + sh.stride_f;
+    unsigned short* id = reinterpret_cast<unsigned short*>(ys + sh.stride_d);
+    unsigned short* jf = id + static_cast<size_t>(sh.stride_d) * sh.len_d;
+    double vx[R], px[R], vpx[R], d1x[R], d2x[R], sx[R], vy[R], py[R], vpy[R], d1y[R], d2y[R], sy[R];
+    int ln_d[R], ln_f[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = tid + i * NT;
+        ln_d[i] = ln_f[i] = 0;
+        vx[i] = px[i] = vpx[i] = d1x[i] = d2x[i] = sx[i] = vy[i] = py[i] = vpy[i] = d1y[i] = d2y[i] = sy[i] = 0.0;
+        if (r < nd) {
+            const int p0 = a.A.ptr[d0 + r];
+            ln_d[i] = a.A.ptr[d0 + r + 1] - p0;
+            for (int e = 0; e < ln_d[i]; ++e) {
+                vd[e * sh.stride_d + r] = a.A.val[p0 + e];
+                id[e * sh.stride_d + r] = static_cast<unsigned short>(a.A.idx[p0 + e] - f0);
+            }
+            vy[i] = a.v.vy[d0 + r];
+            ys[r] = vy[i];
+        }
+        if (r < nf) {
+            const int p0 = a.AT.ptr[f0 + r];
+            ln_f[i] = a.AT.ptr[f0 + r + 1] - p0;
+            for (int e = 0; e < ln_f[i]; ++e) {
+                vf[e * sh.stride_f + r] = a.AT.val[p0 + e];
+                jf[e * sh.stride_f + r] = static_cast<unsigned short>(a.AT.idx[p0 + e] - d0);
+            }
+            vx[i] = a.v.vx[f0 + r];
+            xs[r] = vx[i];
+        }
+    }
+    if (tid == 0) done = 0;
+    MrState s = *sp;  // advanced by thread 0
+    double beta = s.beta;
+    // p_r of mr_rows: the even and the odd entries' sums, then their sum
+    auto row = [](const double* v, const unsigned short* j, int stride, int r, int len, const double* g) {
+        double t0 = 0.0, t1 = 0.0;
+        v += r;
+        j += r;
+        int e = 0;
+#pragma unroll 2
+        for (; e + 1 < len; e += 2, v += 2 * stride, j += 2 * stride) {
+            t0 += v[0] * g[j[0]];
+            t1 += v[stride] * g[j[stride]];
+        }
+        if (e < len) t0 += v[0] * g[j[0]];
+        return t0 + t1;
+    };
+    auto part = [&](double v, double* out) {
+        const double t = warp_sum(v);
+        if ((tid & 31) == 0) out[tid >> 5] = t;
+    };
+    auto total = [&](const double* in) {  // the warps in order
+        double u = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) u += in[w];
+        return u;
+    };
+    __syncthreads();
+    for (;;) {
+        double v = 0.0, v2 = 0.0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + i * NT;
+            py[i] = r < nd ? row(vd, id, sh.stride_d, r, ln_d[i], xs) : 0.0;
+            px[i] = r < nf ? row(vf, jf, sh.stride_f, r, ln_f[i], ys) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (tid + i * NT < nf) v += vx[i] * px[i];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (tid + i * NT < nd) v += vy[i] * py[i];
+        part(v, red);
+        __syncthreads();
+        const double alpha = total(red);
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (tid + i * NT < nf) {
+                px[i] = px[i] - alpha * vx[i] - beta * vpx[i];
+                v2 += px[i] * px[i];
+            }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (tid + i * NT < nd) {
+                py[i] = py[i] - alpha * vy[i] - beta * vpy[i];
+                v2 += py[i] * py[i];
+            }
+        part(v2, red2);
+        __syncthreads();
+        if (tid == 0) mr_scalars(s, alpha, total(red2), bc, &done);
+        __syncthreads();
+        const double phi = bc[1], ig = bc[2], oldeps = bc[3], delta = bc[4], ib = bc[5];
+        beta = bc[0];
+        const bool stop = done != 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = tid + i * NT;
+            if (r < nf) {
+                const double w = (vx[i] - oldeps * d2x[i] - delta * d1x[i]) * ig;
+                d2x[i] = d1x[i];
+                d1x[i] = w;
+                sx[i] += phi * w;
+                vpx[i] = vx[i];
+                vx[i] = px[i] * ib;
+                xs[r] = vx[i];
+            }
+            if (r < nd) {
+                const double w = (vy[i] - oldeps * d2y[i] - delta * d1y[i]) * ig;
+                d2y[i] = d1y[i];
+                d1y[i] = w;
+                sy[i] += phi * w;
+                vpy[i] = vy[i];
+                vy[i] = py[i] * ib;
+                ys[r] = vy[i];
+            }
+        }
+        if (stop) break;
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = tid + i * NT;
+        if (r < nf) a.v.sx[f0 + r] = sx[i];
+        if (r < nd) a.v.sy[d0 + r] = sy[i];
+    }
+    if (tid == 0) *sp = s;
 }
 
 // Per instance: (free columns, dual-active rows) of the codes, one CTA each.
@@ -887,7 +1061,21 @@ struct Diff {
             widest = std::max<long long>(widest, (b_ptr_h[mr_doff_h[k + 1]] - b_ptr_h[mr_doff_h[k]]) +
                                                      (bt_ptr_h[mr_foff_h[k + 1]] - bt_ptr_h[mr_foff_h[k]]));
         const bool one_launch = mr_one_launch_enabled() && widest <= kMrOneLaunchNnz;
-        if (one_launch) {
+        MrChipShape chip{0, 0, 0, 0};  // of the widest instance
+        for (int k = 0; k < p.count; ++k) {
+            chip.stride_d = std::max(chip.stride_d, mr_doff_h[k + 1] - mr_doff_h[k]);
+            chip.stride_f = std::max(chip.stride_f, mr_foff_h[k + 1] - mr_foff_h[k]);
+        }
+        for (int r = 0; r < nd; ++r) chip.len_d = std::max(chip.len_d, b_ptr_h[r + 1] - b_ptr_h[r]);
+        for (int r = 0; r < nf; ++r) chip.len_f = std::max(chip.len_f, bt_ptr_h[r + 1] - bt_ptr_h[r]);
+        const int rows = std::max(chip.stride_d, chip.stride_f);
+        chip.stride_d = (chip.stride_d + 31) & ~31;
+        chip.stride_f = (chip.stride_f + 31) & ~31;
+        if (one_launch && rows <= 2 * kMrSolveThreads && chip.bytes() <= kMrChipSmem) {
+            auto kernel = rows <= kMrSolveThreads ? k_mr_solve_chip<1> : k_mr_solve_chip<2>;
+            GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMrChipSmem)));
+            kernel<<<p.count, kMrSolveThreads, chip.bytes(), s>>>(oa, chip);
+        } else if (one_launch) {
             k_mr_solve<<<p.count, kMrSolveThreads, 0, s>>>(oa);
         } else if (host_loop_mode()) {  // the same steps from the host, one state read-back per chunk
             for (;;) {
