@@ -180,7 +180,7 @@ EXPORTS = [
     "gb_vec_from_host", "gb_vec_to_host", "gb_vec_size", "gb_vec_destroy", "gb_copy", "gb_fill", "gb_spmv_A",
     "gb_spmv_AT", "gb_spmv_Q", "gb_primal_step", "gb_dual_step", "gb_sub", "gb_scale_into", "gb_primal_res2",
     "gb_dual_res", "gb_row_dual_obj", "gb_dot", "gb_dot_c", "gb_diff2", "gb_batch_create", "gb_batch_solve",
-    "gb_batch_get_solution", "gb_batch_schedule", "gb_batch_autotune", "gb_batch_time_kernels", "gb_batch_destroy",
+    "gb_batch_get_solution", "gb_batch_get_solutions", "gb_batch_schedule", "gb_batch_autotune", "gb_batch_time_kernels", "gb_batch_destroy",
     "gb_diff_create", "gb_diff_forward",
     "gb_diff_default_options", "gb_diff_set_options", "gb_diff_backward", "gb_diff_get_info", "gb_diff_tail_start", "gb_diff_destroy",
     "gb_eval_kkt_noalloc", "gb_read_mps", "gb_model_lp", "gb_model_name", "gb_model_free", "gb_factor_detect",
@@ -222,7 +222,8 @@ def load_library(path: str = LIB_PATH):
         "gb_dual_res": (i32, [vp, vp, vp, i32, vp, vp]), "gb_row_dual_obj": (i32, [vp, vp, vp]),
         "gb_dot": (i32, [vp, vp, vp, vp]), "gb_dot_c": (i32, [vp, vp, vp]), "gb_diff2": (i32, [vp, vp, vp, vp]),
         "gb_batch_create": (i32, [i32, vp, vp, vp]), "gb_batch_solve": (i32, [vp, vp, vp]),
-        "gb_batch_get_solution": (i32, [vp, i32, vp, vp]), "gb_batch_schedule": (i32, [vp, vp, vp, vp]),
+        "gb_batch_get_solution": (i32, [vp, i32, vp, vp]), "gb_batch_get_solutions": (i32, [vp, vp, vp]),
+        "gb_batch_schedule": (i32, [vp, vp, vp, vp]),
         "gb_batch_autotune": (i32, [vp, i32, vp, vp, vp, vp]),
         "gb_batch_load_modes": (i32, [vp, vp]), "gb_problem_load_modes": (i32, [vp, vp]),
         "gb_batch_time_kernels": (i32, [vp, i32, i32, vp, vp, vp, vp]),
@@ -628,13 +629,14 @@ class BatchSolver:
         o = _opts(opt)
         res = (_GbResult * len(self.lps))()
         _check(self._lib.gb_batch_solve(self._h, C.addressof(o), res))
-        out = []
-        for i, r in enumerate(res):
-            x = y = None
-            if fetch:
-                x, y = self.solution(i)
-            out.append(_result(r, x, y))
-        return out
+        if not fetch:
+            return [_result(r, None, None) for r in res]
+        # one copy of all points; the results hold their parts of it
+        n = np.cumsum([0] + [lp.n for lp in self.lps])
+        m = np.cumsum([0] + [lp.m for lp in self.lps])
+        x, y = np.empty(int(n[-1])), np.empty(int(m[-1]))
+        _check(self._lib.gb_batch_get_solutions(self._h, _p(x), _p(y)))
+        return [_result(r, x[n[i]:n[i + 1]], y[m[i]:m[i + 1]]) for i, r in enumerate(res)]
 
     def set_start(self, i: int, x=None, y=None) -> None:
         """Warm start of instance i (gb_batch_set_start)."""

@@ -829,13 +829,13 @@ void ensure_resident(Problem& P) {
         int best = 8;
         ResClass c;
         c.cluster = kResMaxCluster;
-        c.threads = 1024;
+        c.threads = 512;
         c.nctas = kResMaxCluster;
         c.smem = kResMaxSmem;
         cudaLaunchAttribute attr[1];
         const cudaLaunchConfig_t cfg = resident_config(c, attr, P.stream);
         int got = 0;
-        if (cudaOccupancyMaxActiveClusters(&got, resident_kernel<V, V>(1024), &cfg) == cudaSuccess && got > 0)
+        if (cudaOccupancyMaxActiveClusters(&got, resident_kernel<V, V>(512), &cfg) == cudaSuccess && got > 0)
             best = kResMaxCluster;
         cudaGetLastError();
         most_cluster[w].store(best);
@@ -2089,6 +2089,16 @@ int gb_batch_get_solution(gb_batch* b, int i, double* x_out, double* y_out) {
         if (y_out && r1 > r0)
             GB_CUDA(cudaMemcpyAsync(y_out, P.yo.get() + r0, sizeof(double) * (r1 - r0), cudaMemcpyDeviceToHost,
                                     P.stream));
+        GB_CUDA(cudaStreamSynchronize(P.stream));
+    });
+}
+
+int gb_batch_get_solutions(gb_batch* b, double* x_out, double* y_out) {
+    return guarded([&] {
+        GB_REQUIRE(b != nullptr && b->p->solved, "no solution available");
+        Problem& P = *b->p;
+        if (x_out) P.xo.download(x_out, P.n, P.stream);
+        if (y_out) P.yo.download(y_out, P.m, P.stream);
         GB_CUDA(cudaStreamSynchronize(P.stream));
     });
 }

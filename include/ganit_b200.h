@@ -309,6 +309,9 @@ int gb_batch_create(int count, const gb_lp* lps, const gb_options* opt, gb_batch
 int gb_batch_solve(gb_batch* b, const gb_options* opt, gb_result* results);
 /* Unscaled solution of instance i (either buffer may be NULL). */
 int gb_batch_get_solution(gb_batch* b, int i, double* x_out, double* y_out);
+/* Unscaled solutions of all instances, concatenated in instance order: one
+ * copy a side instead of two and a wait per instance. */
+int gb_batch_get_solutions(gb_batch* b, double* x_out, double* y_out);
 /* Schedule chosen by the autotuner: threads per block, blocks per SM, and
  * the row-split group sizes picked per instance (written to groups[count*2]
  * when groups != NULL: group size for A rows, for A^T rows). */
