@@ -425,7 +425,7 @@ __device__ __forceinline__ void step_sizes(SolveState& s) {  // pdhg_impl.hpp:87
 }
 
 // Scalar decision logic of one instance, after its partials are reduced.
-static __device__ void decide(SolveState& s, const double (&T)[kTerms], int mode) {
+static __device__ __forceinline__ void decide(SolveState& s, const double (&T)[kTerms], int mode) {
     const Kkt kc = make_kkt(s, T[T_CX_C], T[T_XQX_C], T[T_ROBJ_C], T[T_VOBJ_C], T[T_RP2_C], T[T_RD2_C]);
     if (mode == kEvalCertify) { s.kcert = kc; return; }
     if (mode == kEvalInit) {  // pdhg_impl.hpp:120-128
@@ -597,10 +597,14 @@ __global__ void __launch_bounds__(kThreads) k_decide(const __grid_constant__ Eva
         for (int q = kRowTerms; q < kTerms; ++q)
             for (int b = t0 + first; b < t1; b += step) T[q] += __ldcg(a.partials + q * nb + b);
     };
-    auto finish = [&](SolveState& s, const double (&T)[kTerms]) {
+    // The decision works on a copy of the state: its fields arrive in one round
+    // of independent loads instead of one L2 access after another.
+    auto finish = [&](SolveState& st, const double (&T)[kTerms]) {
+        SolveState s = st;
         s.ran_body = (a.mode == kEvalCheck) ? 1 : 0;
         decide(s, T, a.mode);
         any_active |= s.active;
+        st = s;
     };
     constexpr int kWide = kDecideWide;
     for (int k = k0; k < k1; ++k) {
@@ -625,16 +629,31 @@ __global__ void __launch_bounds__(kThreads) k_decide(const __grid_constant__ Eva
         }
         __syncthreads();
     }
-    for (int k = k0 + wid; k < k1; k += kWarps) {
-        const int nblk = (a.seg_a[k + 1] - a.seg_a[k]) + (a.seg_t[k + 1] - a.seg_t[k]);
-        if (nblk > kWide || !eval_includes(a.st[k], a.mode)) continue;
-        double T[kTerms];
-        load_terms(k, lane, 32, T);
+    // (instance, term) pairs over the warps, kPairs at a time so that their
+    // loads are in flight together (one warp per instance folded its 22 terms
+    // one after another: 11 us for a lone LP)
+    constexpr int kPairs = 4;
+    const int pairs = (k1 - k0) * kTerms;
+    for (int p0 = wid * kPairs; p0 < pairs; p0 += kWarps * kPairs) {
+        double v[kPairs];
 #pragma unroll
-        for (int q = 0; q < kTerms; ++q) T[q] = warp_sum(T[q]);
+        for (int u = 0; u < kPairs; ++u) {
+            v[u] = 0.0;
+            const int p = p0 + u, k = k0 + p / kTerms, q = p % kTerms;
+            if (p >= pairs) continue;
+            const int nblk = (a.seg_a[k + 1] - a.seg_a[k]) + (a.seg_t[k + 1] - a.seg_t[k]);
+            if (nblk > kWide || !eval_includes(a.st[k], a.mode)) continue;
+            const size_t nb = static_cast<size_t>(nbA + a.AT.nb);
+            const int b0 = q < kRowTerms ? a.seg_a[k] : nbA + a.seg_t[k];
+            const int b1 = q < kRowTerms ? a.seg_a[k + 1] : nbA + a.seg_t[k + 1];
+            for (int b = b0 + lane; b < b1; b += 32) v[u] += __ldcg(a.partials + q * nb + b);
+        }
+#pragma unroll
+        for (int u = 0; u < kPairs; ++u) v[u] = warp_sum(v[u]);
         if (lane == 0) {
 #pragma unroll
-            for (int q = 0; q < kTerms; ++q) a.inst_terms[static_cast<size_t>(k) * kTerms + q] = T[q];
+            for (int u = 0; u < kPairs; ++u)
+                if (p0 + u < pairs) a.inst_terms[static_cast<size_t>(k0) * kTerms + p0 + u] = v[u];
         }
     }
     __syncthreads();

@@ -162,6 +162,17 @@ __device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, __nv_bfloat16& a
     a = v.x; b = v.y;
 }
 
+// Sum over the group of 2^lg lanes, into its first lane (reduce_rows' tree).
+template <class V>
+__device__ __forceinline__ V group_tree(V acc, int lg) {
+    if (lg > 4) acc += __shfl_down_sync(0xffffffffu, acc, 16);
+    if (lg > 3) acc += __shfl_down_sync(0xffffffffu, acc, 8);
+    if (lg > 2) acc += __shfl_down_sync(0xffffffffu, acc, 4);
+    if (lg > 1) acc += __shfl_down_sync(0xffffffffu, acc, 2);
+    if (lg > 0) acc += __shfl_down_sync(0xffffffffu, acc, 1);
+    return acc;
+}
+
 // Row sums of a slice: a lane's part over its steps, then the group's tree
 // (the sum lands in each group's first lane).
 template <class M, class V>
@@ -178,13 +189,52 @@ __device__ __forceinline__ V slice_sum(int pair0, int np, int lg, const unsigned
         acc += static_cast<V>(a) * g[j & 0xffffu];
         acc += static_cast<V>(b) * g[j >> 16];
     }
-    if (lg > 4) acc += __shfl_down_sync(0xffffffffu, acc, 16);
-    if (lg > 3) acc += __shfl_down_sync(0xffffffffu, acc, 8);
-    if (lg > 2) acc += __shfl_down_sync(0xffffffffu, acc, 4);
-    if (lg > 1) acc += __shfl_down_sync(0xffffffffu, acc, 2);
-    if (lg > 0) acc += __shfl_down_sync(0xffffffffu, acc, 1);
-    return acc;
+    return group_tree(acc, lg);
 }
+
+// A slice of up to kResRegPairs pairs held in registers across a launch: its
+// sums read shared memory for the gathers alone (a pair's positions and values
+// are 3 of its ~10.7 wavefronts in FP32, 5 of ~18 in FP64).  Pairs past the end
+// are padding (the zero slot with value 0).  For CTAs of 256 threads: LP
+// 701 x 1753 3.74 -> 3.25 ms; with 512 threads it costs the second CTA per SM
+// (37 LPs 2.86 -> 3.3 ms) and gains nothing where the exchange is the longer
+// part (LP 2000 x 5000).
+constexpr int kResRegPairs = 8;
+template <class M>
+struct RegSlice {
+    unsigned j[kResRegPairs];
+    M v[2 * kResRegPairs];
+    __device__ __forceinline__ void load(const ResSlice& e, const unsigned* idx, const M* val, unsigned zero, int lane) {
+        const int np = e.meta & 0xff;
+#pragma unroll
+        for (int t = 0; t < kResRegPairs; ++t) {
+            j[t] = zero;
+            v[2 * t] = v[2 * t + 1] = static_cast<M>(0.0f);
+            if (t < np) {
+                j[t] = idx[(e.pair0 + t) * 32 + lane];
+                ld_pair(val + (e.pair0 + t) * 64 + 2 * lane, v[2 * t], v[2 * t + 1]);
+            }
+        }
+    }
+    template <class V>
+    __device__ __forceinline__ V sum(int np, int lg, const V* g) const {
+        V acc = V(0);
+#pragma unroll
+        for (int h = 0; h < kResRegPairs; h += 4) {
+            if (h < np) {
+                V x[8];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    x[2 * t] = g[j[h + t] & 0xffffu];
+                    x[2 * t + 1] = g[j[h + t] >> 16];
+                }
+#pragma unroll
+                for (int t = 0; t < 8; ++t) acc += static_cast<V>(v[2 * h + t]) * x[t];
+            }
+        }
+        return group_tree(acc, lg);
+    }
+};
 
 template <class M, class V>
 struct ResArgs {
@@ -204,7 +254,7 @@ struct ResArgs {
 };
 
 template <class M, class V, int T>
-__global__ void __launch_bounds__(T) k_resident(const __grid_constant__ ResArgs<M, V> a) {
+__global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_constant__ ResArgs<M, V> a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const ResCta r = a.cta[blockIdx.x];
     const SolveState& s = a.st[r.inst];
@@ -279,13 +329,28 @@ __global__ void __launch_bounds__(T) k_resident(const __grid_constant__ ResArgs<
     };
     if (a.cluster > 1) cluster_sync();  // every CTA has started and holds its share
     else __syncthreads();
+    // each warp's first slice of either side in registers
+    RegSlice<M> reg_t, reg_a;
+    bool has_t = false, has_a = false;
+    constexpr bool kReg = T <= 256;  // larger CTAs keep 64 registers a thread, so that two share an SM
+    if (kReg && warp < r.ns_t) {
+        const ResSlice e = sl[warp];
+        has_t = (e.meta & 0xff) <= kResRegPairs;
+        if (has_t) reg_t.load(e, idx, val, static_cast<unsigned>(r.m) * 0x10001u, lane);
+    }
+    if (kReg && warp < r.ns_a) {
+        const ResSlice e = sl[r.ns_t + warp];
+        has_a = (e.meta & 0xff) <= kResRegPairs;
+        if (has_a) reg_a.load(e, idx, val, static_cast<unsigned>(r.n) * 0x10001u, lane);
+    }
     for (int it = 0; it < a.iters; ++it) {
         for (int q = warp; q < r.ns_t; q += W) {  // primal half (PrimalEpi)
             const ResSlice e = sl[q];
             const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
             const int k = e.own0 + grp;
             const V xk = ox[k], ck = oc[k], lk = ol[k], uk = ou[k], sk = osx[k];
-            const V t = slice_sum<M, V>(e.pair0, np, lg, idx, val, ys, lane);
+            const V t = kReg && q == warp && has_t ? reg_t.template sum<V>(np, lg, ys)
+                                           : slice_sum<M, V>(e.pair0, np, lg, idx, val, ys, lane);
             const V g = ck - t + V(0);
             V v = xk - tau * g;
             v = (v < lk) ? lk : v;
@@ -302,7 +367,8 @@ __global__ void __launch_bounds__(T) k_resident(const __grid_constant__ ResArgs<
             const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
             const int k = e.own0 + grp;
             const V yk = ys[e.pos0 + grp], sk = osy[k], lk = sigma * olo[k], hk = sigma * ohi[k];
-            const V t = slice_sum<M, V>(e.pair0, np, lg, idx, val, xs, lane);
+            const V t = kReg && q == r.ns_t + warp && has_a ? reg_a.template sum<V>(np, lg, xs)
+                                                    : slice_sum<M, V>(e.pair0, np, lg, idx, val, xs, lane);
             const V qv = yk - sigma * t;
             V w = -qv;
             w = (w < lk) ? lk : w;
