@@ -5,7 +5,9 @@
 // src/backend_cuda.cu:286-378, and CpuBackendT<M,R>, src/backend_cpu.cpp:38-156).
 // Matrix products use the row-block SpMV of gb_spmv.cuh; reductions are
 // fixed-order two-pass FP64 sums (the reference uses atomicAdd, so its
-// results vary run to run; these do not).
+// results vary run to run; these do not).  Every kernel is launched with
+// programmatic dependent launch (pdl_enter): a host program's iteration is a
+// chain of four 3-4 us kernels, whose launch gaps it hides.
 #include <cstring>
 #include <memory>
 
@@ -34,6 +36,7 @@ int guarded_b(F&& f) {
 template <class V>
 __global__ void kb_primal_step(int n, const V* x, const V* aty, const V* qx, const V* c, const V* l, const V* u,
                                V tau, V* xn, V* xbar, V* sumx) {
+    pdl_enter();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const V xj = x[j];
         const V g = c[j] - aty[j] + (qx ? qx[j] : V(0));
@@ -48,6 +51,7 @@ __global__ void kb_primal_step(int n, const V* x, const V* aty, const V* qx, con
 template <class V>
 __global__ void kb_dual_step(int m, const V* y, const V* axbar, const V* lo, const V* hi, V sigma, V* yn,
                              V* sumy) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
         const V q = y[i] - sigma * axbar[i];
         const V a = sigma * lo[i], b = sigma * hi[i];
@@ -61,25 +65,30 @@ __global__ void kb_dual_step(int m, const V* y, const V* axbar, const V* lo, con
 }
 template <class V>
 __global__ void kb_sub(int n, const V* a, const V* b, V* d) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) d[i] = a[i] - b[i];
 }
 template <class V>
 __global__ void kb_scale(int n, double a, const V* s, V* d) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         d[i] = static_cast<V>(a * static_cast<double>(s[i]));
 }
 template <class V>
 __global__ void kb_fill(int n, double a, V* d) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) d[i] = static_cast<V>(a);
 }
 template <class V>
 __global__ void kb_to_double(int n, const V* s, double* d) {
+    pdl_enter();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) d[i] = double(s[i]);
 }
 
 // ---- two-channel fixed-order reductions (backend_cpu.cpp:101-155)
 template <class F>
 __global__ void __launch_bounds__(kThreads) kb_red1(int n, F f, double* part) {
+    pdl_enter();
     __shared__ double sh[kWarps * 2];
     double v[2] = {0.0, 0.0};
     for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
@@ -95,6 +104,7 @@ __global__ void __launch_bounds__(kThreads) kb_red1(int n, F f, double* part) {
     }
 }
 __global__ void __launch_bounds__(kThreads) kb_red2(int np, const double* part, double* out) {
+    pdl_enter();
     __shared__ double sh[kWarps * 2];
     double v[2] = {0.0, 0.0};
     for (int i = threadIdx.x; i < np; i += kThreads) {
@@ -185,7 +195,7 @@ struct Backend {
     DevSchedule a_s, at_s, q_s;
     // data in the vector type
     Vec c, l, u, lo, hi, rres, cres;
-    DevBuf<double> part, out;
+    DevBuf<double> part;
     double* out_host = nullptr;
     ~Backend() {
         cudaSetDevice(device);
@@ -242,13 +252,13 @@ void vec_from_host(Backend& B, Vec& v, const double* h, int k) {
 template <class F>
 std::pair<double, double> reduce2(Backend& B, int k, F f) {
     if (k > 0) {
-        kb_red1<F><<<kRedGrid, kThreads, 0, B.stream>>>(k, f, B.part.get());
-        kb_red2<<<1, kThreads, 0, B.stream>>>(kRedGrid, B.part.get(), B.out.get());
+        launch_pdl(kb_red1<F>, kRedGrid, kThreads, 0, B.stream, k, f, B.part.get());
+        // the two sums go straight to the pinned host words
+        launch_pdl(kb_red2, 1, kThreads, 0, B.stream, kRedGrid, static_cast<const double*>(B.part.get()), B.out_host);
+        GB_CUDA(cudaStreamSynchronize(B.stream));
     } else {
-        GB_CUDA(cudaMemsetAsync(B.out.get(), 0, 2 * sizeof(double), B.stream));
+        B.out_host[0] = B.out_host[1] = 0.0;
     }
-    GB_CUDA(cudaMemcpyAsync(B.out_host, B.out.get(), 2 * sizeof(double), cudaMemcpyDeviceToHost, B.stream));
-    GB_CUDA(cudaStreamSynchronize(B.stream));
     GB_CUDA(cudaGetLastError());
     return {B.out_host[0], B.out_host[1]};
 }
@@ -262,8 +272,8 @@ void spmv_t(Backend& B, int which, const Vec& x, Vec& y) {
     const int rows = which == 0 ? B.m : B.n;
     if (rows == 0 || s.nb == 0) return;
     static_assert(spmv_smem_bytes<1, double>() <= 48 * 1024, "single-vector SpMV fits the default smem limit");
-    k_spmv<M, V><<<s.nb, kThreads, spmv_smem_bytes<1, V>(), B.stream>>>(bview<M>(ptr, idx, val, s, rows), x.p<V>(),
-                                                                     y.p<V>());
+    launch_pdl(k_spmv<M, V>, s.nb, kThreads, spmv_smem_bytes<1, V>(), B.stream, bview<M>(ptr, idx, val, s, rows),
+               static_cast<const V*>(x.p<V>()), y.p<V>());
     GB_CUDA(cudaGetLastError());
 }
 
@@ -342,7 +352,6 @@ int gb_backend_create(const gb_scaled_lp* s, int mat_type, int vec_type, gb_back
         vec_from_host(B, B.hi, s->hi, s->m);
         vec_from_host(B, B.rres, s->rres, s->m);
         B.part.reset(2 * kRedGrid);
-        B.out.reset(2);
         B.out_host = static_cast<double*>(host_alloc(2 * sizeof(double)));
         GB_CUDA(cudaStreamSynchronize(B.stream));
         *out = h.release();
@@ -379,7 +388,7 @@ int gb_vec_to_host(gb_backend* b, const gb_vec* v, double* h) {
         const int k = v->v.k;
         if (!k) return;
         DevBuf<double> tmp(k);
-        GB_DISPATCH_V(B, kb_to_double<V><<<elem_grid(k, B.sms), kThreads, 0, B.stream>>>(k, v->v.p<V>(), tmp.get()));
+        GB_DISPATCH_V(B, launch_pdl(kb_to_double<V>, elem_grid(k, B.sms), kThreads, 0, B.stream, k, static_cast<const V*>(v->v.p<V>()), tmp.get()));
         tmp.download(h, k, B.stream);
         GB_CUDA(cudaStreamSynchronize(B.stream));
     });
@@ -401,7 +410,7 @@ int gb_fill(gb_backend* b, gb_vec* v, double a) {
     return guarded_b([&] {
         GB_REQUIRE(b && v, "bad arguments");
         Backend& B = b->b;
-        if (v->v.k) GB_DISPATCH_V(B, kb_fill<V><<<elem_grid(v->v.k, B.sms), kThreads, 0, B.stream>>>(v->v.k, a, v->v.p<V>()));
+        if (v->v.k) GB_DISPATCH_V(B, launch_pdl(kb_fill<V>, elem_grid(v->v.k, B.sms), kThreads, 0, B.stream, v->v.k, a, v->v.p<V>()));
     });
 }
 
@@ -427,9 +436,12 @@ int gb_primal_step(gb_backend* b, const gb_vec* x, const gb_vec* aty, const gb_v
         GB_REQUIRE(b && x && aty && xn && xbar && sumx, "bad arguments");
         Backend& B = b->b;
         const int n = B.n;
-        GB_DISPATCH_V(B, kb_primal_step<V><<<elem_grid(n, B.sms), kThreads, 0, B.stream>>>(
-                             n, x->v.p<V>(), aty->v.p<V>(), qx ? qx->v.p<V>() : nullptr, B.c.p<V>(), B.l.p<V>(),
-                             B.u.p<V>(), static_cast<V>(tau), xn->v.p<V>(), xbar->v.p<V>(), sumx->v.p<V>()));
+        GB_DISPATCH_V(B, const V* q = qx ? qx->v.p<V>() : nullptr;
+                      launch_pdl(kb_primal_step<V>, elem_grid(n, B.sms), kThreads, 0, B.stream, n,
+                                 static_cast<const V*>(x->v.p<V>()), static_cast<const V*>(aty->v.p<V>()), q,
+                                 static_cast<const V*>(B.c.p<V>()), static_cast<const V*>(B.l.p<V>()),
+                                 static_cast<const V*>(B.u.p<V>()), static_cast<V>(tau), xn->v.p<V>(),
+                                 xbar->v.p<V>(), sumx->v.p<V>()));
     });
 }
 
@@ -438,9 +450,10 @@ int gb_dual_step(gb_backend* b, const gb_vec* y, const gb_vec* axbar, double sig
         GB_REQUIRE(b && y && axbar && yn && sumy, "bad arguments");
         Backend& B = b->b;
         const int m = B.m;
-        GB_DISPATCH_V(B, kb_dual_step<V><<<elem_grid(m, B.sms), kThreads, 0, B.stream>>>(
-                             m, y->v.p<V>(), axbar->v.p<V>(), B.lo.p<V>(), B.hi.p<V>(), static_cast<V>(sigma),
-                             yn->v.p<V>(), sumy->v.p<V>()));
+        GB_DISPATCH_V(B, launch_pdl(kb_dual_step<V>, elem_grid(m, B.sms), kThreads, 0, B.stream, m,
+                                    static_cast<const V*>(y->v.p<V>()), static_cast<const V*>(axbar->v.p<V>()),
+                                    static_cast<const V*>(B.lo.p<V>()), static_cast<const V*>(B.hi.p<V>()),
+                                    static_cast<V>(sigma), yn->v.p<V>(), sumy->v.p<V>()));
     });
 }
 
@@ -449,7 +462,7 @@ int gb_sub(gb_backend* b, const gb_vec* a, const gb_vec* c, gb_vec* d) {
         GB_REQUIRE(b && a && c && d, "bad arguments");
         Backend& B = b->b;
         const int k = a->v.k;
-        if (k) GB_DISPATCH_V(B, kb_sub<V><<<elem_grid(k, B.sms), kThreads, 0, B.stream>>>(k, a->v.p<V>(), c->v.p<V>(), d->v.p<V>()));
+        if (k) GB_DISPATCH_V(B, launch_pdl(kb_sub<V>, elem_grid(k, B.sms), kThreads, 0, B.stream, k, static_cast<const V*>(a->v.p<V>()), static_cast<const V*>(c->v.p<V>()), d->v.p<V>()));
     });
 }
 
@@ -458,7 +471,7 @@ int gb_scale_into(gb_backend* b, const gb_vec* src, double a, gb_vec* dst) {
         GB_REQUIRE(b && src && dst, "bad arguments");
         Backend& B = b->b;
         const int k = src->v.k;
-        if (k) GB_DISPATCH_V(B, kb_scale<V><<<elem_grid(k, B.sms), kThreads, 0, B.stream>>>(k, a, src->v.p<V>(), dst->v.p<V>()));
+        if (k) GB_DISPATCH_V(B, launch_pdl(kb_scale<V>, elem_grid(k, B.sms), kThreads, 0, B.stream, k, a, static_cast<const V*>(src->v.p<V>()), dst->v.p<V>()));
     });
 }
 
