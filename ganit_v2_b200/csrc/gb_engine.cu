@@ -257,6 +257,10 @@ void init_kernel_attrs() {
         init_resident_attrs<__nv_bfloat16, float>();
         init_resident_attrs<float, double>();
         init_resident_attrs<double, double>();
+        set_smem(k_grid<float, float>, kGridSmem);
+        set_smem(k_grid<__nv_bfloat16, float>, kGridSmem);
+        set_smem(k_grid<float, double>, kGridSmem);
+        set_smem(k_grid<double, double>, kGridSmem);
         set_smem(k_qp_chip<float, float>, kQpSmem);
         set_smem(k_qp_chip<float, double>, kQpSmem);
         set_smem(k_qp_chip<double, double>, kQpSmem);
@@ -757,24 +761,28 @@ void launch_resident(Problem& P, VecSet<V>& vs, const ResClass& c, int ce, cudaS
     GB_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel<M, V>(c.threads), a));
 }
 
-// Packed values of matrix type M (made on first use; the structure is there).
+// Packed values of one type (made on first use; the structure is there).
+template <class Buf, class Src>
+void pack_values(Problem& P, Buf& buf, long long pairs, const DevBuf<int>& slot_t, const DevBuf<int>& slot_a,
+                 const DevBuf<ResSliceAt>& at, Src src) {
+    if (buf.get()) return;
+    cudaStream_t s = P.stream;
+    buf.reset(static_cast<size_t>(pairs) * 64);
+    GB_CUDA(cudaMemsetAsync(buf.get(), 0, buf.size() * sizeof(*buf.get()), s));
+    const int gt = elem_grid(P.n, P.sms), ga = elem_grid(P.m, P.sms);
+    k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), slot_t.get(), at.get(), buf.get());
+    k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), slot_a.get(), at.get(), buf.get());
+    GB_CUDA(cudaGetLastError());
+}
+
 template <class M, class V>
 void ensure_resident_values(Problem& P) {
     ResPlan& R = P.res[sizeof(V) == 8];
     if (!R.any()) return;
-    cudaStream_t s = P.stream;
-    auto pack = [&](auto& buf, auto src) {
-        if (buf.get()) return;
-        buf.reset(static_cast<size_t>(R.pairs) * 64);
-        GB_CUDA(cudaMemsetAsync(buf.get(), 0, buf.size() * sizeof(*buf.get()), s));
-        const int gt = elem_grid(P.n, P.sms), ga = elem_grid(P.m, P.sms);
-        k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), R.slot_t.get(), R.at.get(), buf.get());
-        k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), R.slot_a.get(), R.at.get(), buf.get());
-    };
+    auto pack = [&](auto& buf, auto src) { pack_values(P, buf, R.pairs, R.slot_t, R.slot_a, R.at, src); };
     if constexpr (std::is_same<M, double>::value) pack(R.val64, [](const DevMat& A) { return A.val64.get(); });
     else if constexpr (std::is_same<M, float>::value) pack(R.val32, [](const DevMat& A) { return A.val32.get(); });
     else pack(R.valbf, [](const DevMat& A) { return A.valbf.get(); });
-    GB_CUDA(cudaGetLastError());
 }
 
 // Which instances run on chip with vectors of type V (index w), in clusters
@@ -1028,11 +1036,247 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     GB_CUDA(cudaLaunchKernelEx(&cfg, k_qp_chip<M, V>, a));
 }
 
+// A single LP that no cluster holds, kept by the whole GPU (k_grid): rows all
+// STREAM rows, each CTA's gathered entries within 16-bit positions, and its
+// vectors, gathered entries and at least half of the matrix in shared memory.
+// (Below that the matrix streams from L2 anyway, and eight streaming CTAs per
+// SM read it faster than one.)
+template <class V>
+void build_grid(Problem& P, GridPlan& R) {
+    constexpr int w = sizeof(V) == 8;
+    constexpr size_t pair_bytes = 128 + 64 * sizeof(V);
+    constexpr int kMaxVector = 2 << 20;  // the packing's bitmaps: 148 vectors of bits
+    if (P.count != 1 || P.has_q || P.res[w].any() || P.sms < kGridCtas || !resident_enabled() ||
+        std::max(P.n, P.m) > kMaxVector || P.A.nnz < 1 ||
+        static_cast<double>(P.A.nnz) / 32.0 * static_cast<double>(pair_bytes) > 2.0 * kGridCtas * kGridSmem)
+        return;
+    cudaStream_t s = P.stream;
+    const DevMat* mats[2] = {&P.AT, &P.A};
+    const DevSchedule* sched[2] = {&P.AT.template sched_for<V>(), &P.A.template sched_for<V>()};
+    std::vector<ResSide> sides[2];
+    std::vector<ResSliceAt> at;
+    std::vector<ResSlice> slices;
+    std::vector<GridCta> cta(kGridCtas);
+    std::vector<std::vector<ResSlice>> mine[2];
+    long long pairs = 0;
+    for (int sd = 0; sd < 2; ++sd) {
+        const int rows = mats[sd]->rows;
+        const int* ptr = mats[sd]->host_ptr.data();
+        std::vector<unsigned char> lg(rows);
+        for (const RowBlock& b : sched[sd]->host_blocks) {
+            if (b.kind != kStream) return;
+            for (int r = b.r0; r < b.r1; ++r) lg[r] = static_cast<unsigned char>(w ? res_lg64(ptr[r + 1] - ptr[r]) : b.lg);
+        }
+        // contiguous shares of equal nonzeros + 4 per row (its epilogue)
+        const double total = static_cast<double>(ptr[rows]) + 4.0 * rows;
+        mine[sd].resize(kGridCtas);
+        int r = 0;
+        for (int c = 0; c < kGridCtas; ++c) {
+            const double end = total * (c + 1) / kGridCtas;
+            ResSide S{};
+            S.row0 = S.at0 = r;
+            ResHist H;
+            while (r < rows && (c == kGridCtas - 1 || ptr[r + 1] + 4.0 * (r + 1) <= end)) {
+                const int len = ptr[r + 1] - ptr[r], steps = (len + (1 << lg[r]) - 1) >> lg[r];
+                if (steps > kResMaxSteps) return;
+                ++H.h[lg[r]][(steps + 1) >> 1];
+                ++r;
+            }
+            S.row1 = r;
+            for (int g = 0; g < 6; ++g) {
+                int run = 0;
+                for (int b = kResBins - 1; b >= 0; --b) {
+                    S.rank0[g][b] = run;
+                    run += H.h[g][b];
+                }
+                S.slice0[g] = -1;
+            }
+            // slices by falling pairs; their pairs lie in that order
+            struct Item {
+                int lg, pairs, rows;
+            };
+            std::vector<Item> it;
+            H.each_slice([&](int g, int np, int nr) { it.push_back({g, np, nr}); });
+            std::vector<int> order(it.size());
+            std::iota(order.begin(), order.end(), 0);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return it[x].pairs > it[y].pairs; });
+            std::vector<ResSliceAt> place(it.size());
+            int own = 0, pair = 0;
+            for (int k : order) {
+                const Item& e = it[k];
+                const int meta = e.pairs | e.lg << 8 | e.rows << 12;
+                mine[sd][c].push_back({pair, meta, own, own});
+                place[k] = {pairs + pair, meta, own};
+                own += e.rows;
+                pair += e.pairs;
+            }
+            for (size_t k = 0; k < it.size(); ++k)
+                if (S.slice0[it[k].lg] < 0) S.slice0[it[k].lg] = static_cast<int>(at.size() + k);
+            at.insert(at.end(), place.begin(), place.end());
+            (sd == 0 ? cta[c].pair_t0 : cta[c].pair_a0) = pairs;
+            (sd == 0 ? cta[c].pos_t0 : cta[c].pos_a0) = S.row0;
+            (sd == 0 ? cta[c].own_t : cta[c].own_a) = own;
+            pairs += pair;
+            sides[sd].push_back(S);
+        }
+    }
+    auto put = [&](auto& d, const auto& h) {
+        d.reset(std::max<size_t>(h.size(), 1));
+        d.upload(h.data(), h.size(), s);
+    };
+    put(R.at, at);
+    std::vector<int> count[2], list0[2];
+    for (int sd = 0; sd < 2; ++sd) {
+        const int rows = mats[sd]->rows, words = div_up(mats[sd]->cols, 32);
+        put(R.sides[sd], sides[sd]);
+        R.src[sd].reset(rows);
+        R.slot[sd].reset(rows);
+        R.pos[sd].reset(rows);
+        if (w == 0) {
+            R.lg[sd].reset(rows);
+            k_res_row_lg<<<sched[sd]->nb, kThreads, 0, s>>>(sched[sd]->nb, sched[sd]->blocks.get(), R.lg[sd].get());
+        }
+        k_res_rank<<<kGridCtas, 32, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), R.lg[sd].get(), R.at.get(),
+                                            R.slot[sd].get(), nullptr, R.src[sd].get());
+        k_grid_inverse<<<elem_grid(rows, P.sms), kThreads, 0, s>>>(rows, R.src[sd].get(), R.pos[sd].get());
+        R.bits[sd].reset(static_cast<size_t>(kGridCtas) * words);
+        R.before[sd].reset(static_cast<size_t>(kGridCtas) * words);
+        R.count[sd].reset(kGridCtas);
+        GB_CUDA(cudaMemsetAsync(R.bits[sd].get(), 0, sizeof(unsigned) * R.bits[sd].size(), s));
+        k_grid_mark<<<kGridCtas, 1024, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), mats[sd]->idx.get(), words,
+                                               R.bits[sd].get(), R.before[sd].get(), R.count[sd].get());
+        count[sd].resize(kGridCtas);
+        R.count[sd].download(count[sd].data(), kGridCtas, s);
+    }
+    GB_CUDA(cudaStreamSynchronize(s));
+    GB_CUDA(cudaGetLastError());
+    for (int sd = 0; sd < 2; ++sd) {
+        list0[sd].assign(kGridCtas + 1, 0);
+        for (int c = 0; c < kGridCtas; ++c) {
+            if (count[sd][c] >= kResMaxIndex) return;
+            list0[sd][c + 1] = list0[sd][c] + count[sd][c];
+        }
+    }
+    // what each CTA keeps in shared memory
+    long long kept = 0;
+    for (int c = 0; c < kGridCtas; ++c) {
+        GridCta& k = cta[c];
+        k.u_t = count[0][c];
+        k.u_a = count[1][c];
+        k.list_t0 = list0[0][c];
+        k.list_a0 = list0[1][c];
+        k.ns_t = static_cast<int>(mine[0][c].size());
+        k.ns_a = static_cast<int>(mine[1][c].size());
+        k.slice0 = static_cast<int>(slices.size());
+        const size_t fixed = grid_fixed_bytes<V>(k);
+        if (fixed > kGridSmem) return;
+        long long budget = static_cast<long long>((kGridSmem - fixed) / pair_bytes), all = 0;
+        for (int sd = 0; sd < 2; ++sd)
+            for (const ResSlice& e : mine[sd][c]) all += e.meta & 0xff;
+        for (int sd = 0; sd < 2; ++sd) {
+            long long side = 0, got = 0;
+            for (const ResSlice& e : mine[sd][c]) side += e.meta & 0xff;
+            const long long most = all <= budget ? side : budget * side / all;
+            int res = 0;
+            for (const ResSlice& e : mine[sd][c]) {
+                if (got + (e.meta & 0xff) > most) break;
+                got += e.meta & 0xff;
+                ++res;
+            }
+            (sd == 0 ? k.res_t : k.res_a) = res;
+            (sd == 0 ? k.pairs_t : k.pairs_a) = static_cast<int>(got);
+            kept += got;
+            slices.insert(slices.end(), mine[sd][c].begin(), mine[sd][c].end());
+        }
+        R.smem = std::max(R.smem, fixed + pair_bytes * (k.pairs_t + k.pairs_a));
+    }
+    if (2 * kept < pairs) return;
+    R.pairs = pairs;
+    put(R.cta, cta);
+    put(R.slices, slices);
+    R.idx.reset(std::max<size_t>(static_cast<size_t>(pairs) * 32, 1));
+    R.gx.reset(P.n);
+    R.gy.reset(P.m);
+    R.sync.reset(2);
+    GB_CUDA(cudaMemsetAsync(R.sync.get(), 0, 2 * sizeof(unsigned), s));
+    for (int sd = 0; sd < 2; ++sd) {
+        const int words = div_up(mats[sd]->cols, 32);
+        std::vector<long long> p0(kGridCtas + 1);
+        for (int c = 0; c < kGridCtas; ++c) p0[c] = sd == 0 ? cta[c].pair_t0 : cta[c].pair_a0;
+        p0[kGridCtas] = sd == 0 ? cta[0].pair_a0 : pairs;
+        put(R.pair0[sd], p0);
+        put(R.list0[sd], list0[sd]);
+        R.list[sd].reset(std::max(list0[sd][kGridCtas], 1));
+        k_grid_lists<<<kGridCtas, kThreads, 0, s>>>(words, R.bits[sd].get(), R.before[sd].get(), R.list0[sd].get(),
+                                                    R.pos[1 - sd].get(), R.list[sd].get());
+        k_grid_fill<<<kGridCtas, kThreads, 0, s>>>(R.sides[sd].get(), R.pair0[sd].get(), R.count[sd].get(), R.idx.get());
+        k_grid_entries<<<kGridCtas, 1024, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), mats[sd]->idx.get(),
+                                                  R.slot[sd].get(), R.at.get(), words, R.bits[sd].get(),
+                                                  R.before[sd].get(), reinterpret_cast<unsigned short*>(R.idx.get()));
+    }
+    GB_CUDA(cudaGetLastError());
+    R.on = true;
+    if (trace_enabled())
+        std::fprintf(stderr, "[gb trace] grid f%d: %lld of %lld pairs on chip, %d + %d gathered, %zu B\n", w ? 64 : 32,
+                     kept, pairs, list0[0][kGridCtas], list0[1][kGridCtas], R.smem);
+}
+
+template <class V>
+void ensure_grid(Problem& P) {
+    GridPlan& R = P.grid[sizeof(V) == 8];
+    if (R.built) return;
+    build_grid<V>(P, R);
+    if (!R.on) R = GridPlan{};
+    R.built = true;
+}
+
+template <class M>
+const M* grid_values(const GridPlan& R);
+template <>
+const float* grid_values<float>(const GridPlan& R) { return R.val32.get(); }
+template <>
+const double* grid_values<double>(const GridPlan& R) { return R.val64.get(); }
+template <>
+const __nv_bfloat16* grid_values<__nv_bfloat16>(const GridPlan& R) { return R.valbf.get(); }
+
+template <class M, class V>
+void ensure_grid_values(Problem& P) {
+    GridPlan& R = P.grid[sizeof(V) == 8];
+    if (!R.on) return;
+    if constexpr (std::is_same<M, double>::value) pack_values(P, R.val64, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.val64.get(); });
+    else if constexpr (std::is_same<M, float>::value) pack_values(P, R.val32, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.val32.get(); });
+    else pack_values(P, R.valbf, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.valbf.get(); });
+}
+
+template <class M, class V>
+void launch_grid(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
+    const GridPlan& R = P.grid[sizeof(V) == 8];
+    const bool odd = (ce & 1) != 0;
+    GridArgs<M, V> a{R.cta.get(), R.slices.get(), R.idx.get(), grid_values<M>(R), R.list[0].get(), R.list[1].get(),
+                     R.src[0].get(), R.src[1].get(), reinterpret_cast<V*>(R.gx.get()), reinterpret_cast<V*>(R.gy.get()),
+                     vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(), odd ? vs.y1.get() : vs.y0.get(),
+                     vs.sumx.get(), vs.sumy.get(), vs.c.get(), vs.l.get(), vs.u.get(), vs.lo.get(), vs.hi.get(),
+                     P.st.get(), R.sync.get(), P.phase_flags.get() + P.count, ce};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(kGridCtas);
+    cfg.blockDim = dim3(kGridThreads);
+    cfg.dynamicSmemBytes = R.smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeCooperative;  // its CTAs wait for one another
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GB_CUDA(cudaLaunchKernelEx(&cfg, k_grid<M, V>, a));
+}
+
 // What a body of level <M, V> needs on chip; before its graph is captured.
 template <class M, class V>
 void prepare_resident(Problem& P) {
     ensure_resident<V>(P);
     ensure_resident_values<M, V>(P);
+    ensure_grid<V>(P);
+    ensure_grid_values<M, V>(P);
     if (P.dplr && !P.qp_sync.get()) {
         P.qp_sync.reset(2);
         GB_CUDA(cudaMemsetAsync(P.qp_sync.get(), 0, 2 * sizeof(unsigned), P.stream));
@@ -1136,7 +1380,11 @@ long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cuda
         launch_resident<M, V>(P, vs, c, ce, s);
         ++nl;
     }
-    bool on_chip = false;
+    bool on_chip = P.grid[sizeof(V) == 8].on;
+    if (on_chip) {
+        launch_grid<M, V>(P, vs, ce, s);
+        ++nl;
+    }
     if constexpr (!std::is_same<M, __nv_bfloat16>::value)  // the BF16 level takes LPs only
         if (qp_on_chip<M, V>(P)) {
             launch_qp_chip<M, V>(P, vs, ce, s);
@@ -1696,6 +1944,7 @@ void rebuild_schedules(Problem& P, int w) {
     GB_CUDA(cudaStreamSynchronize(s));
     for (auto& g : P.graphs) g.reset();
     for (ResPlan& r : P.res) r = ResPlan{};  // packed by these schedules' lanes per row
+    for (GridPlan& r : P.grid) r = GridPlan{};
     P.qp_at_lg.release();
     DevSchedule& sa = w == 0 ? P.A.sched32 : P.A.sched;
     DevSchedule& st = w == 0 ? P.AT.sched32 : P.AT.sched;

@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "../../include/ganit_b200.h"
+#include "gb_grid.cuh"
 #include "gb_pdhg.cuh"
 #include "gb_qp_chip.cuh"
 #include "gb_resident.cuh"
@@ -150,6 +151,7 @@ struct Problem {
     DevBuf<unsigned char> qp_at_lg;       // k_qp_chip: log2 lanes per row of A^T (FP32)
     DevBuf<unsigned> qp_sync;             // k_qp_chip's {arrivals, exits}
     DevBuf<double> qp_slots;              // and its row sums
+    GridPlan grid[2];                     // a single LP kept by the whole GPU: FP32 vectors, FP64 vectors
     ResPlan res[2];                       // instances iterated on chip: FP32 vectors, FP64 vectors
     double setup_seconds = 0.0;
     long long launches = 0;               // kernel launches of the last solve

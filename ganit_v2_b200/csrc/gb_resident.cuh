@@ -453,7 +453,7 @@ static __global__ void k_res_rank(const ResSide* __restrict__ sides, const int* 
             const int e = sd.slice0[lg] + k / rows, grp = k % rows;
             const int p = slices[e].pos0 + grp;
             slot[r] = e * 32 + grp;
-            pos[r] = static_cast<unsigned short>(p);
+            if (pos) pos[r] = static_cast<unsigned short>(p);
             at[sd.at0 + p] = r;
         }
     }
