@@ -652,7 +652,7 @@ template <class M, class V>
 StreamBlocks stream_blocks(const Problem& P) {
     const ResPlan& R = P.res[sizeof(V) == 8];
     if (P.list_level == level_index<M, V>()) return {P.list_a.get(), P.list_t.get(), P.list_na, P.list_nt};
-    if (R.any()) return {R.list_a.get(), R.list_t.get(), R.list_na, R.list_nt};
+    if (R.any()) return {R.list_a, R.list_t, R.list_na, R.list_nt};
     return {};
 }
 
@@ -752,8 +752,8 @@ template <class M, class V>
 void launch_resident(Problem& P, VecSet<V>& vs, const ResClass& c, int ce, cudaStream_t s) {
     const ResPlan& R = P.res[sizeof(V) == 8];
     const bool odd = (ce & 1) != 0;
-    ResArgs<M, V> a{R.cta.get() + c.cta0, R.slices.get(), R.idx.get(), resident_values<M>(R), R.col_at.get(),
-                    R.row_at.get(), vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(),
+    ResArgs<M, V> a{R.cta + c.cta0, R.slices, R.idx, resident_values<M>(R), R.col_at,
+                    R.row_at, vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(),
                     odd ? vs.y1.get() : vs.y0.get(), vs.sumx.get(), vs.sumy.get(), vs.c.get(), vs.l.get(),
                     vs.u.get(), vs.lo.get(), vs.hi.get(), P.st.get(), P.phase_flags.get() + P.count, ce, c.cluster};
     cudaLaunchAttribute attr[1];
@@ -763,15 +763,15 @@ void launch_resident(Problem& P, VecSet<V>& vs, const ResClass& c, int ce, cudaS
 
 // Packed values of one type (made on first use; the structure is there).
 template <class Buf, class Src>
-void pack_values(Problem& P, Buf& buf, long long pairs, const DevBuf<int>& slot_t, const DevBuf<int>& slot_a,
-                 const DevBuf<ResSliceAt>& at, Src src) {
+void pack_values(Problem& P, Buf& buf, long long pairs, const int* slot_t, const int* slot_a, const ResSliceAt* at,
+                 Src src) {
     if (buf.get()) return;
     cudaStream_t s = P.stream;
     buf.reset(static_cast<size_t>(pairs) * 64);
     GB_CUDA(cudaMemsetAsync(buf.get(), 0, buf.size() * sizeof(*buf.get()), s));
     const int gt = elem_grid(P.n, P.sms), ga = elem_grid(P.m, P.sms);
-    k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), slot_t.get(), at.get(), buf.get());
-    k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), slot_a.get(), at.get(), buf.get());
+    k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), slot_t, at, buf.get());
+    k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), slot_a, at, buf.get());
     GB_CUDA(cudaGetLastError());
 }
 
@@ -908,47 +908,6 @@ void ensure_resident(Problem& P) {
     }
     R.pairs = T.pairs;
     cudaStream_t s = P.stream;
-    auto put = [&](auto& d, const auto& h) {
-        d.reset(std::max<size_t>(h.size(), 1));
-        d.upload(h.data(), h.size(), s);
-    };
-    put(R.cta, T.cta);
-    put(R.slices, T.slices);
-    put(R.at, T.at);
-    auto &d_t = R.sides_t, &d_a = R.sides_a;
-    put(d_t, T.sides[0]);
-    put(d_a, T.sides[1]);
-    R.idx.reset(std::max<size_t>(static_cast<size_t>(T.pairs) * 32, 1));
-    R.col_at.reset(T.positions[0]);
-    R.row_at.reset(T.positions[1]);
-    GB_CUDA(cudaMemsetAsync(R.col_at.get(), 0xff, sizeof(int) * T.positions[0], s));
-    GB_CUDA(cudaMemsetAsync(R.row_at.get(), 0xff, sizeof(int) * T.positions[1], s));
-    R.slot_t.reset(P.n);
-    R.slot_a.reset(P.m);
-    auto &pos_t = R.pos_t, &pos_a = R.pos_a;
-    auto &lg_t = R.lg_t, &lg_a = R.lg_a;
-    pos_t.reset(P.n);
-    pos_a.reset(P.m);
-    GB_CUDA(cudaMemsetAsync(R.slot_t.get(), 0xff, sizeof(int) * P.n, s));
-    GB_CUDA(cudaMemsetAsync(R.slot_a.get(), 0xff, sizeof(int) * P.m, s));
-    if (w == 0) {
-        lg_t.reset(P.n);
-        lg_a.reset(P.m);
-        k_res_row_lg<<<st.nb, kThreads, 0, s>>>(st.nb, st.blocks.get(), lg_t.get());
-        k_res_row_lg<<<sa.nb, kThreads, 0, s>>>(sa.nb, sa.blocks.get(), lg_a.get());
-    }
-    const int ns = static_cast<int>(placed.size());
-    k_res_rank<<<ns, 32, 0, s>>>(d_t.get(), P.AT.ptr.get(), lg_t.get(), R.at.get(), R.slot_t.get(), pos_t.get(),
-                                 R.col_at.get());
-    k_res_rank<<<ns, 32, 0, s>>>(d_a.get(), P.A.ptr.get(), lg_a.get(), R.at.get(), R.slot_a.get(), pos_a.get(),
-                                 R.row_at.get());
-    k_res_fill<<<static_cast<int>(T.cta.size()), kThreads, 0, s>>>(R.cta.get(), R.idx.get());
-    unsigned short* idx16 = reinterpret_cast<unsigned short*>(R.idx.get());
-    k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t.get(),
-                                                             R.at.get(), pos_a.get(), idx16);
-    k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a.get(),
-                                                             R.at.get(), pos_t.get(), idx16);
-    GB_CUDA(cudaGetLastError());
     std::vector<RowBlock> la, lt;
     for (int k = 0; k < P.count; ++k) {
         if (R.resident[k]) continue;
@@ -957,8 +916,40 @@ void ensure_resident(Problem& P) {
     }
     R.list_na = static_cast<int>(la.size());
     R.list_nt = static_cast<int>(lt.size());
-    put(R.list_a, la);
-    put(R.list_t, lt);
+    PlanArena arena;
+    arena.host(R.cta, T.cta);
+    arena.host(R.slices, T.slices);
+    arena.host(R.at, T.at);
+    arena.host(R.sides_t, T.sides[0]);
+    arena.host(R.sides_a, T.sides[1]);
+    arena.host(R.list_a, la);
+    arena.host(R.list_t, lt);
+    arena.ones(R.col_at, T.positions[0]);
+    arena.ones(R.row_at, T.positions[1]);
+    arena.ones(R.slot_t, P.n);
+    arena.ones(R.slot_a, P.m);
+    arena.raw(R.idx, static_cast<size_t>(T.pairs) * 32);
+    arena.raw(R.pos_t, P.n);
+    arena.raw(R.pos_a, P.m);
+    if (w == 0) {
+        arena.raw(R.lg_t, P.n);
+        arena.raw(R.lg_a, P.m);
+    }
+    arena.commit(R.mem, P.pinned, s);
+    if (w == 0) {
+        k_res_row_lg<<<st.nb, kThreads, 0, s>>>(st.nb, st.blocks.get(), R.lg_t);
+        k_res_row_lg<<<sa.nb, kThreads, 0, s>>>(sa.nb, sa.blocks.get(), R.lg_a);
+    }
+    const int ns = static_cast<int>(placed.size());
+    k_res_rank<<<ns, 32, 0, s>>>(R.sides_t, P.AT.ptr.get(), R.lg_t, R.at, R.slot_t, R.pos_t, R.col_at);
+    k_res_rank<<<ns, 32, 0, s>>>(R.sides_a, P.A.ptr.get(), R.lg_a, R.at, R.slot_a, R.pos_a, R.row_at);
+    k_res_fill<<<static_cast<int>(T.cta.size()), kThreads, 0, s>>>(R.cta, R.idx);
+    unsigned short* idx16 = reinterpret_cast<unsigned short*>(R.idx);
+    k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t, R.at,
+                                                             R.pos_a, idx16);
+    k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a, R.at,
+                                                             R.pos_t, idx16);
+    GB_CUDA(cudaGetLastError());
     if (trace_enabled())
         for (const ResClass& c : R.classes)
             std::fprintf(stderr, "[gb trace] resident f%d: %d CTAs in clusters of %d, %d threads, %zu B\n", w ? 64 : 32,
@@ -1047,9 +1038,11 @@ void build_grid(Problem& P, GridPlan& R) {
     constexpr size_t pair_bytes = 128 + 64 * sizeof(V);
     constexpr int kMaxVector = 2 << 20;  // the packing's bitmaps: 148 vectors of bits
     if (P.count != 1 || P.has_q || P.res[w].any() || P.sms < kGridCtas || !resident_enabled() ||
-        std::max(P.n, P.m) > kMaxVector || P.A.nnz < 1 ||
-        static_cast<double>(P.A.nnz) / 32.0 * static_cast<double>(pair_bytes) > 2.0 * kGridCtas * kGridSmem)
+        std::max(P.n, P.m) > kMaxVector || P.A.nnz < 1)
         return;
+    // before any work: the vectors and half of the matrix against the GPU's shared memory
+    const double room = static_cast<double>(kGridCtas) * kGridSmem - sizeof(V) * (5.0 * P.n + 4.0 * P.m);
+    if (static_cast<double>(P.A.nnz) / 32.0 * static_cast<double>(pair_bytes) > 2.0 * room) return;
     cudaStream_t s = P.stream;
     const DevMat* mats[2] = {&P.AT, &P.A};
     const DevSchedule* sched[2] = {&P.AT.template sched_for<V>(), &P.A.template sched_for<V>()};
@@ -1120,33 +1113,33 @@ void build_grid(Problem& P, GridPlan& R) {
             sides[sd].push_back(S);
         }
     }
-    auto put = [&](auto& d, const auto& h) {
-        d.reset(std::max<size_t>(h.size(), 1));
-        d.upload(h.data(), h.size(), s);
-    };
-    put(R.at, at);
+    PlanArena first;
+    first.host(R.at, at);
+    for (int sd = 0; sd < 2; ++sd) {
+        const size_t rows = mats[sd]->rows, map = static_cast<size_t>(kGridCtas) * div_up(mats[sd]->cols, 32);
+        first.host(R.sides[sd], sides[sd]);
+        first.raw(R.src[sd], rows);
+        first.raw(R.slot[sd], rows);
+        first.raw(R.pos[sd], rows);
+        if (w == 0) first.raw(R.lg[sd], rows);
+        first.raw(R.bits[sd], map);
+        first.raw(R.before[sd], map);
+        first.raw(R.count[sd], kGridCtas);
+    }
+    first.commit(R.mem[0], P.pinned, s);
     std::vector<int> count[2], list0[2];
     for (int sd = 0; sd < 2; ++sd) {
         const int rows = mats[sd]->rows, words = div_up(mats[sd]->cols, 32);
-        put(R.sides[sd], sides[sd]);
-        R.src[sd].reset(rows);
-        R.slot[sd].reset(rows);
-        R.pos[sd].reset(rows);
-        if (w == 0) {
-            R.lg[sd].reset(rows);
-            k_res_row_lg<<<sched[sd]->nb, kThreads, 0, s>>>(sched[sd]->nb, sched[sd]->blocks.get(), R.lg[sd].get());
-        }
-        k_res_rank<<<kGridCtas, 32, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), R.lg[sd].get(), R.at.get(),
-                                            R.slot[sd].get(), nullptr, R.src[sd].get());
-        k_grid_inverse<<<elem_grid(rows, P.sms), kThreads, 0, s>>>(rows, R.src[sd].get(), R.pos[sd].get());
-        R.bits[sd].reset(static_cast<size_t>(kGridCtas) * words);
-        R.before[sd].reset(static_cast<size_t>(kGridCtas) * words);
-        R.count[sd].reset(kGridCtas);
-        GB_CUDA(cudaMemsetAsync(R.bits[sd].get(), 0, sizeof(unsigned) * R.bits[sd].size(), s));
-        k_grid_mark<<<kGridCtas, 1024, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), mats[sd]->idx.get(), words,
-                                               R.bits[sd].get(), R.before[sd].get(), R.count[sd].get());
+        if (w == 0)
+            k_res_row_lg<<<sched[sd]->nb, kThreads, 0, s>>>(sched[sd]->nb, sched[sd]->blocks.get(), R.lg[sd]);
+        k_res_rank<<<kGridCtas, 32, 0, s>>>(R.sides[sd], mats[sd]->ptr.get(), R.lg[sd], R.at, R.slot[sd], nullptr,
+                                            R.src[sd]);
+        k_grid_inverse<<<elem_grid(rows, P.sms), kThreads, 0, s>>>(rows, R.src[sd], R.pos[sd]);
+        GB_CUDA(cudaMemsetAsync(R.bits[sd], 0, sizeof(unsigned) * kGridCtas * words, s));
+        k_grid_mark<<<kGridCtas, 1024, 0, s>>>(R.sides[sd], mats[sd]->ptr.get(), mats[sd]->idx.get(), words, R.bits[sd],
+                                               R.before[sd], R.count[sd]);
         count[sd].resize(kGridCtas);
-        R.count[sd].download(count[sd].data(), kGridCtas, s);
+        GB_CUDA(cudaMemcpyAsync(count[sd].data(), R.count[sd], sizeof(int) * kGridCtas, cudaMemcpyDeviceToHost, s));
     }
     GB_CUDA(cudaStreamSynchronize(s));
     GB_CUDA(cudaGetLastError());
@@ -1192,27 +1185,34 @@ void build_grid(Problem& P, GridPlan& R) {
     }
     if (2 * kept < pairs) return;
     R.pairs = pairs;
-    put(R.cta, cta);
-    put(R.slices, slices);
-    R.idx.reset(std::max<size_t>(static_cast<size_t>(pairs) * 32, 1));
-    R.gx.reset(P.n);
-    R.gy.reset(P.m);
-    R.sync.reset(2);
-    GB_CUDA(cudaMemsetAsync(R.sync.get(), 0, 2 * sizeof(unsigned), s));
+    std::vector<long long> p0[2];
+    for (int sd = 0; sd < 2; ++sd) {
+        p0[sd].resize(kGridCtas + 1);
+        for (int c = 0; c < kGridCtas; ++c) p0[sd][c] = sd == 0 ? cta[c].pair_t0 : cta[c].pair_a0;
+        p0[sd][kGridCtas] = sd == 0 ? cta[0].pair_a0 : pairs;
+    }
+    PlanArena second;
+    second.host(R.cta, cta);
+    second.host(R.slices, slices);
+    for (int sd = 0; sd < 2; ++sd) {
+        second.host(R.pair0[sd], p0[sd]);
+        second.host(R.list0[sd], list0[sd]);
+        second.raw(R.list[sd], list0[sd][kGridCtas]);
+    }
+    second.raw(R.idx, static_cast<size_t>(pairs) * 32);
+    second.raw(R.gx, P.n);
+    second.raw(R.gy, P.m);
+    second.raw(R.sync, 2);
+    second.commit(R.mem[1], P.pinned, s);
+    GB_CUDA(cudaMemsetAsync(R.sync, 0, 2 * sizeof(unsigned), s));
     for (int sd = 0; sd < 2; ++sd) {
         const int words = div_up(mats[sd]->cols, 32);
-        std::vector<long long> p0(kGridCtas + 1);
-        for (int c = 0; c < kGridCtas; ++c) p0[c] = sd == 0 ? cta[c].pair_t0 : cta[c].pair_a0;
-        p0[kGridCtas] = sd == 0 ? cta[0].pair_a0 : pairs;
-        put(R.pair0[sd], p0);
-        put(R.list0[sd], list0[sd]);
-        R.list[sd].reset(std::max(list0[sd][kGridCtas], 1));
-        k_grid_lists<<<kGridCtas, kThreads, 0, s>>>(words, R.bits[sd].get(), R.before[sd].get(), R.list0[sd].get(),
-                                                    R.pos[1 - sd].get(), R.list[sd].get());
-        k_grid_fill<<<kGridCtas, kThreads, 0, s>>>(R.sides[sd].get(), R.pair0[sd].get(), R.count[sd].get(), R.idx.get());
-        k_grid_entries<<<kGridCtas, 1024, 0, s>>>(R.sides[sd].get(), mats[sd]->ptr.get(), mats[sd]->idx.get(),
-                                                  R.slot[sd].get(), R.at.get(), words, R.bits[sd].get(),
-                                                  R.before[sd].get(), reinterpret_cast<unsigned short*>(R.idx.get()));
+        k_grid_lists<<<kGridCtas, kThreads, 0, s>>>(words, R.bits[sd], R.before[sd], R.list0[sd], R.pos[1 - sd],
+                                                    R.list[sd]);
+        k_grid_fill<<<kGridCtas, kThreads, 0, s>>>(R.pair0[sd], R.count[sd], R.idx);
+        k_grid_entries<<<kGridCtas, 1024, 0, s>>>(R.sides[sd], mats[sd]->ptr.get(), mats[sd]->idx.get(), R.slot[sd],
+                                                  R.at, words, R.bits[sd], R.before[sd],
+                                                  reinterpret_cast<unsigned short*>(R.idx));
     }
     GB_CUDA(cudaGetLastError());
     R.on = true;
@@ -1252,11 +1252,11 @@ template <class M, class V>
 void launch_grid(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     const GridPlan& R = P.grid[sizeof(V) == 8];
     const bool odd = (ce & 1) != 0;
-    GridArgs<M, V> a{R.cta.get(), R.slices.get(), R.idx.get(), grid_values<M>(R), R.list[0].get(), R.list[1].get(),
-                     R.src[0].get(), R.src[1].get(), reinterpret_cast<V*>(R.gx.get()), reinterpret_cast<V*>(R.gy.get()),
+    GridArgs<M, V> a{R.cta, R.slices, R.idx, grid_values<M>(R), R.list[0], R.list[1],
+                     R.src[0], R.src[1], reinterpret_cast<V*>(R.gx), reinterpret_cast<V*>(R.gy),
                      vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(), odd ? vs.y1.get() : vs.y0.get(),
                      vs.sumx.get(), vs.sumy.get(), vs.c.get(), vs.l.get(), vs.u.get(), vs.lo.get(), vs.hi.get(),
-                     P.st.get(), R.sync.get(), P.phase_flags.get() + P.count, ce};
+                     P.st.get(), R.sync, P.phase_flags.get() + P.count, ce};
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(kGridCtas);

@@ -277,30 +277,30 @@ static __global__ void k_grid_inverse(int k, const int* __restrict__ at, int* __
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) pos[at[q]] = q;
 }
 // Padding of a CTA's pairs: the zero slot after its gathered entries.
-static __global__ void k_grid_fill(const ResSide* __restrict__ sides, const long long* __restrict__ pair0,
-                                   const int* __restrict__ count, unsigned* __restrict__ idx) {
+static __global__ void k_grid_fill(const long long* __restrict__ pair0, const int* __restrict__ count, unsigned* __restrict__ idx) {
     const unsigned z = static_cast<unsigned>(count[blockIdx.x]) * 0x10001u;
     for (long long k = 32 * pair0[blockIdx.x] + threadIdx.x; k < 32 * pair0[blockIdx.x + 1]; k += blockDim.x) idx[k] = z;
 }
 
 struct GridPlan {
     bool built = false, on = false;
-    DevBuf<GridCta> cta;
-    DevBuf<ResSlice> slices;
-    DevBuf<ResSliceAt> at;
-    DevBuf<ResSide> sides[2];
-    DevBuf<unsigned> idx;
+    DevBuf<unsigned char> mem[2];                  // everything below but the values
+    GridCta* cta = nullptr;
+    ResSlice* slices = nullptr;
+    ResSliceAt* at = nullptr;
+    ResSide* sides[2] = {};                        // A^T, A
+    int *list[2] = {}, *src[2] = {}, *slot[2] = {}, *pos[2] = {};
+    unsigned* bits[2] = {};                        // packing scratch
+    int *before[2] = {}, *count[2] = {}, *list0[2] = {};
+    unsigned char* lg[2] = {};
+    long long* pair0[2] = {};
+    unsigned* idx = nullptr;
+    double *gx = nullptr, *gy = nullptr;           // xbar / y by packed position
+    unsigned* sync = nullptr;
     DevBuf<float> val32;
     DevBuf<double> val64;
     DevBuf<__nv_bfloat16> valbf;
-    DevBuf<int> list[2], src[2], slot[2], pos[2];  // A^T, A
-    DevBuf<unsigned> bits[2];                      // packing scratch
-    DevBuf<int> before[2], count[2], list0[2];
-    DevBuf<long long> pair0[2];
     size_t smem = 0;
-    DevBuf<unsigned char> lg[2];
-    DevBuf<double> gx, gy;                         // xbar / y by packed position
-    DevBuf<unsigned> sync;
     long long pairs = 0;
 };
 

@@ -651,26 +651,75 @@ struct ResTables {
     }
 };
 
+// Device arrays of a plan in one allocation (a cudaMalloc each took longer
+// than packing a small LP), those filled by the host in one copy, those that
+// start as -1 in one memset.  The copy's source is pinned, so the host goes on
+// while earlier work of the stream runs; the caller frees it (host_free) with
+// the problem.
+class PlanArena {
+   public:
+    template <class T>
+    void host(T*& p, const std::vector<T>& v) {
+        add(reinterpret_cast<void**>(&p), v.size() * sizeof(T), 0, v.data());
+    }
+    template <class T>
+    void ones(T*& p, size_t n) { add(reinterpret_cast<void**>(&p), n * sizeof(T), 1, nullptr); }
+    template <class T>
+    void raw(T*& p, size_t n) { add(reinterpret_cast<void**>(&p), n * sizeof(T), 2, nullptr); }
+    void commit(DevBuf<unsigned char>& mem, std::vector<void*>& pinned, cudaStream_t s) {
+        size_t end[3], off = 0;
+        for (int kind = 0; kind < 3; ++kind) {
+            for (Item& i : items_)
+                if (i.kind == kind) {
+                    i.off = off;
+                    off += (i.bytes + 255) & ~size_t(255);
+                }
+            end[kind] = off;
+        }
+        mem.reset(std::max<size_t>(off, 256));
+        unsigned char* stage = static_cast<unsigned char*>(host_alloc(std::max<size_t>(end[0], 1)));
+        pinned.push_back(stage);
+        for (const Item& i : items_) {
+            *i.slot = mem.get() + i.off;
+            if (i.kind == 0 && i.bytes) std::memcpy(stage + i.off, i.src, i.bytes);
+        }
+        mem.upload(stage, end[0], s);
+        if (end[1] > end[0]) GB_CUDA(cudaMemsetAsync(mem.get() + end[0], 0xff, end[1] - end[0], s));
+    }
+
+   private:
+    struct Item {
+        void** slot;
+        size_t bytes;
+        int kind;
+        const void* src;
+        size_t off;
+    };
+    std::vector<Item> items_;
+    void add(void** slot, size_t bytes, int kind, const void* src) { items_.push_back({slot, bytes, kind, src, 0}); }
+};
+
 // The resident instances of a problem for one vector precision.
 struct ResPlan {
     bool built = false;
     std::vector<char> resident;             // per instance
     std::vector<ResClass> classes;
-    DevBuf<ResCta> cta;
-    DevBuf<ResSlice> slices;
-    DevBuf<unsigned> idx;
+    DevBuf<unsigned char> mem;              // everything below but the values
+    ResCta* cta = nullptr;
+    ResSlice* slices = nullptr;
+    ResSliceAt* at = nullptr;
+    ResSide *sides_t = nullptr, *sides_a = nullptr;
+    unsigned* idx = nullptr;
+    int *col_at = nullptr, *row_at = nullptr, *slot_t = nullptr, *slot_a = nullptr;
+    unsigned short *pos_t = nullptr, *pos_a = nullptr;
+    unsigned char *lg_t = nullptr, *lg_a = nullptr;
     DevBuf<float> val32;
     DevBuf<double> val64;
     DevBuf<__nv_bfloat16> valbf;
-    DevBuf<int> col_at, row_at, slot_t, slot_a;
-    DevBuf<ResSliceAt> at;
-    DevBuf<ResSide> sides_t, sides_a;       // packing scratch, freed with the plan
-    DevBuf<unsigned short> pos_t, pos_a;
-    DevBuf<unsigned char> lg_t, lg_a;
     long long pairs = 0;
     // Row blocks of the other instances, which the streaming kernels run
     // (nothing: every instance is resident).
-    DevBuf<RowBlock> list_a, list_t;
+    RowBlock *list_a = nullptr, *list_t = nullptr;
     int list_na = 0, list_nt = 0;
     bool any() const { return !classes.empty(); }
 };
