@@ -173,6 +173,13 @@ void inst_reduce(Problem& P, bool rows, F f, int slot, Post post, cudaStream_t s
 // A'^T A', scaling.cpp:108-124 for Q').
 void qx_dplr_f64(Problem& P, const double* x, double* out, cudaStream_t s);
 
+constexpr int kPowerIters = 50;
+void prepare_power(Problem& P);
+void launch_power_chip(Problem& P, cudaStream_t s);
+bool all_resident(const Problem& P) {
+    const ResPlan& R = P.res[1];
+    return R.any() && R.list_na == 0;
+}
 void power_iteration(Problem& P, bool q, cudaStream_t s) {
     const int n = P.n;
     double* v = P.x64.get();  // FP64 vectors double as scratch before the solve
@@ -180,12 +187,15 @@ void power_iteration(Problem& P, bool q, cudaStream_t s) {
     double* z = P.work1.get();
     double* sc = P.scal.get();
     const int gi = div_up(P.count, kThreads);
-    k_fill<<<elem_grid(n, P.sms), kThreads, 0, s>>>(n, 1.0, v);
-    inst_reduce(P, false, Sq{v}, S_PW_NORM, PostSqrt{}, s);
-    k_power_reset<<<gi, kThreads, 0, s>>>(P.count, sc);
-    k_power_vec<<<elem_grid(n, P.sms), kThreads, 0, s>>>(n, P.icol(), sc, v, v, 0);  // v /= ||v||
+    const bool chip = !q && all_resident(P);
+    if (!chip) {
+        k_fill<<<elem_grid(n, P.sms), kThreads, 0, s>>>(n, 1.0, v);
+        inst_reduce(P, false, Sq{v}, S_PW_NORM, PostSqrt{}, s);
+        k_power_reset<<<gi, kThreads, 0, s>>>(P.count, sc);
+        k_power_vec<<<elem_grid(n, P.sms), kThreads, 0, s>>>(n, P.icol(), sc, v, v, 0);  // v /= ||v||
+    }
     const size_t sm1 = spmv_smem_bytes<1, double>();
-    const int iters = q ? 60 : 50;
+    const int iters = q ? 60 : chip ? 0 : kPowerIters;
     for (int it = 0; it < iters; ++it) {
         if (q) {
             if (P.dplr) qx_dplr_f64(P, v, z, s);
@@ -200,6 +210,7 @@ void power_iteration(Problem& P, bool q, cudaStream_t s) {
         launch_pdl(k_power_vec, elem_grid(n, P.sms), kThreads, 0, s, n, P.icol(), sc, static_cast<const double*>(z), v,
                    static_cast<int>(P.count));
     }
+    if (!q) launch_power_chip(P, s);
     k_finish_norms<<<gi, kThreads, 0, s>>>(P.count, P.d_nnz_off.get(), sc, q ? 1 : 0);
 }
 
@@ -234,6 +245,7 @@ void convert_data(Problem& P, VecSet<V>& vs, cudaStream_t s) {
 
 template <class M, class V>
 void init_resident_attrs();
+void init_power_attrs();
 
 // Kernels whose dynamic shared memory exceeds the 48 KB default opt in.
 void init_kernel_attrs() {
@@ -253,6 +265,7 @@ void init_kernel_attrs() {
         set_smem(k_dplr_expand<double, 1>, expand_smem_bytes<double, 1>(kMaxRank));
         set_smem(k_dplr_expand<double, 2>, expand_smem_bytes<double, 2>(kMaxRank));
         set_smem(k_spmv_q2<double, double>, spmv_smem_bytes<2, double>());
+        init_power_attrs();
         init_resident_attrs<float, float>();
         init_resident_attrs<__nv_bfloat16, float>();
         init_resident_attrs<float, double>();
@@ -402,6 +415,7 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     GB_CUDA(cudaMemsetAsync(P->red_arrivals.get(), 0, sizeof(unsigned), s));
     P->st.reset(count);
     P->phase_flags.reset(count + 1);
+    GB_CUDA(cudaMemsetAsync(P->phase_flags.get(), 0, sizeof(int) * (count + 1), s));
     GB_CUDA(cudaMemsetAsync(P->st.get(), 0, sizeof(SolveState) * count, s));
 
     // schedules (host, from the row-length histogram, per instance) and transpose
@@ -494,7 +508,10 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
                                                                                   P->F64.get(), P->D64.get());
     }
     if (P->has_q) power_iteration(*P, true, s);
-    power_iteration(*P, false, s);  // ||A'|| (scaling.cpp:131-155)
+    // ||A'|| (scaling.cpp:131-155): on chip for the resident instances, whatever
+    // shares their batch
+    prepare_power(*P);
+    power_iteration(*P, false, s);
     tr.mark("power iteration");
     // w0 from the scaled data (pdhg_impl.hpp:258-261)
     inst_reduce(*P, false, Sq{P->c.get()}, S_CN, PostSqrt{}, s);
@@ -529,8 +546,11 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     P->phase_flags_host = static_cast<int*>(host_alloc(sizeof(int) * (count + 1)));
     tr.mark("pinned state");
     GB_CUDA(cudaMemcpyAsync(P->scal_host.data(), sc, sizeof(double) * P->scal_host.size(), cudaMemcpyDeviceToHost, s));
+    GB_CUDA(cudaMemcpyAsync(P->phase_flags_host + count, P->phase_flags.get() + count, sizeof(int),
+                            cudaMemcpyDeviceToHost, s));
     GB_CUDA(cudaStreamSynchronize(s));
     GB_CUDA(cudaGetLastError());
+    if (P->phase_flags_host[count]) throw Error(GB_ERR_CUDA, "an exchange between the CTAs of a cluster timed out");
     P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return P.release();
 }
@@ -717,6 +737,13 @@ void init_resident_attrs() {
     set(k_resident<M, V, 1024>);
 }
 
+void init_power_attrs() {
+    for (auto kernel : {k_power_chip<256>, k_power_chip<512>, k_power_chip<1024>}) {
+        set_smem(kernel, kResMaxSmem);
+        GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+}
+
 template <class M, class V>
 auto resident_kernel(int threads) {
     return threads == 256 ? k_resident<M, V, 256> : threads == 512 ? k_resident<M, V, 512> : k_resident<M, V, 1024>;
@@ -870,6 +897,8 @@ void ensure_resident(Problem& P) {
             if (static_cast<size_t>(pairs) * (128 + 64 * sm) > C * kResMaxSmem) continue;  // cannot fit
             res_deal(HH, C, p.deal);
             p.smem = p.deal.smem(sm, sizeof(V));
+            if (w)
+                for (const ResCta& c : p.deal.cta) p.smem = std::max(p.smem, power_smem_bytes(c));
             if (p.smem <= kResMaxSmem) break;
         }
         if (C > cmax) continue;
@@ -1025,6 +1054,22 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     GB_CUDA(cudaLaunchKernelEx(&cfg, k_qp_chip<M, V>, a));
+}
+
+// The FP64 plan, ahead of the power iteration that runs on it.
+void prepare_power(Problem& P) {
+    ensure_resident<double>(P);
+    ensure_resident_values<double, double>(P);
+}
+void launch_power_chip(Problem& P, cudaStream_t s) {
+    const ResPlan& R = P.res[1];
+    for (const ResClass& c : R.classes) {
+        const PowerArgs a{R.cta + c.cta0, R.slices, R.idx, R.val64.get(), P.scal.get(), kScal, S_PW_LAMBDA,
+                          P.phase_flags.get() + P.count, kPowerIters, c.cluster};
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = resident_config(c, attr, s);
+        GB_CUDA(cudaLaunchKernelEx(&cfg, c.threads == 256 ? k_power_chip<256> : c.threads == 512 ? k_power_chip<512> : k_power_chip<1024>, a));
+    }
 }
 
 // A single LP that no cluster holds, kept by the whole GPU (k_grid): rows all

@@ -148,6 +148,26 @@ __device__ __forceinline__ void copy_to_peer(const void* p, unsigned bytes, unsi
 // Shared-memory writes of this thread, before a bulk copy reads them.
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// End of a half iteration: this CTA's share `p` of a gathered vector goes to
+// every other CTA of the cluster, and theirs are awaited (`total`: the vector's
+// bytes; `bar`: its mbarrier, at the phase of `parity`).  Returns `lost`, or
+// whether the wait ran out; once lost, later waits are skipped.
+__device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, unsigned total, unsigned long long* bar,
+                                                 unsigned parity, int cluster, int rank, bool lost) {
+    if (cluster == 1) {
+        __syncthreads();
+        return lost;
+    }
+    fence_async_proxy();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        if (lane == 0) mbar_expect(bar, total - bytes);
+        if (lane < cluster && lane != rank && bytes) copy_to_peer(p, bytes, bar, lane);
+    }
+    return lost || !mbar_wait(bar, parity);
+}
+
 // Two matrix values of a lane's step pair.
 __device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
     const float2 v = *reinterpret_cast<const float2*>(p);
@@ -312,20 +332,8 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
     const int rank = static_cast<int>(blockIdx.x) % a.cluster;
     const unsigned bytes_x = sizeof(V) * r4(r.own_t), bytes_y = sizeof(V) * r4(r.own_a);
     bool lost = false;
-    // End of a half: this CTA's share `p` of a gathered vector goes to every
-    // other CTA, and theirs are awaited (total: the vector's bytes).
     auto exchange = [&](const V* p, unsigned bytes, unsigned total, int b, int it) {
-        if (a.cluster == 1) {
-            __syncthreads();
-            return;
-        }
-        fence_async_proxy();
-        __syncthreads();
-        if (warp == 0) {
-            if (lane == 0) mbar_expect(bar + b, total - bytes);
-            if (lane < a.cluster && lane != rank && bytes) copy_to_peer(p, bytes, bar + b, lane);
-        }
-        if (!lost) lost = !mbar_wait(bar + b, it & 1);
+        lost = cluster_exchange(p, bytes, total, bar + b, it & 1, a.cluster, rank, lost);
     };
     if (a.cluster > 1) cluster_sync();  // every CTA has started and holds its share
     else __syncthreads();
@@ -396,6 +404,89 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
         a.sumy[i] = osy[k];
     }
     if (a.cluster > 1) cluster_sync();  // no CTA leaves while a copy may still read its share
+}
+
+// Power iteration on A'^T A' (scaling.cpp:131-155) of the resident instances on
+// the FP64 plan: 50 steps in one launch instead of 200 launches (0.6 - 1 ms of
+// a small LP's set-up; 0.1 - 0.2 ms here).  z is in xs and w in ys; after z's
+// exchange every CTA forms ||z|| over all of it in the same order.
+inline size_t power_smem_bytes(const ResCta& c) {
+    return res_smem_bytes<double, double>(c.ns_t + c.ns_a, c.pairs, c.n, c.m, 0, 0) + 8 * 32;
+}
+struct PowerArgs {
+    const ResCta* cta;
+    const ResSlice* slices;
+    const unsigned* idx;
+    const double* val;
+    double* scal;          // per instance rows of kScal; [lambda] is written
+    int scal_stride, lambda;
+    int* error;
+    int iters, cluster;
+};
+template <int T>
+__global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid_constant__ PowerArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const ResCta r = a.cta[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int W = T / 32;
+    auto r4 = [](int k) { return (k + 3) & ~3; };
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);
+    double* xs = reinterpret_cast<double*>(smem + kResBarBytes);
+    double* ys = xs + r4(r.n + 1);
+    ResSlice* sl = reinterpret_cast<ResSlice*>(ys + r4(r.m + 1));
+    unsigned* idx = reinterpret_cast<unsigned*>(sl + r.ns_t + r.ns_a);
+    double* val = reinterpret_cast<double*>(idx + 32 * r.pairs);
+    double* red = val + 64 * r.pairs;
+    for (int k = tid; k < r.ns_t + r.ns_a; k += T) cp_async16(sl + k, a.slices + r.slice0 + k);
+    for (int k = tid; k < 8 * r.pairs; k += T) cp_async16(idx + 4 * k, a.idx + 32 * r.pair0 + 4 * k);
+    for (int k = tid; k < 32 * r.pairs; k += T) cp_async16(val + 2 * k, a.val + 64 * r.pair0 + 2 * k);
+    // places between two shares and the zero slots stay 0: they add nothing to ||z||
+    for (int k = tid; k <= r.n; k += T) xs[k] = 0.0;
+    for (int k = tid; k <= r.m; k += T) ys[k] = 0.0;
+    if (tid == 0) {
+        mbar_init(bar);
+        mbar_init(bar + 1);
+        mbar_init_visible();
+    }
+    const int rank = static_cast<int>(blockIdx.x) % a.cluster;
+    const unsigned bytes_x = 8 * r4(r.own_t), bytes_y = 8 * r4(r.own_a);
+    cp_async_wait_all();
+    if (a.cluster > 1) cluster_sync();
+    else __syncthreads();
+    for (int k = tid; k < r.own_t; k += T) xs[r.pos_t0 + k] = 1.0;  // v = 1 / ||1||: the first ||z|| is sqrt(n)
+    bool lost = false;
+    double lambda = 0.0;
+    for (int it = 0; it <= a.iters; ++it) {
+        lost = cluster_exchange(xs + r.pos_t0, bytes_x, 8u * r.n, bar, it & 1, a.cluster, rank, lost);
+        double s = 0.0;
+        for (int k = tid; k < r.n; k += T) s += xs[k] * xs[k];
+        s = warp_sum(s);
+        if (lane == 0) red[warp] = s;
+        __syncthreads();
+        double nz = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) nz += red[w];
+        nz = sqrt(nz);
+        if (it > 0 && nz != 0.0) lambda = nz;
+        if (it == a.iters || nz == 0.0) break;  // the same in every CTA
+        // w = A z / ||z||: z itself stays as it is while peers may still copy it
+        for (int q = r.ns_t + warp; q < r.ns_t + r.ns_a; q += W) {
+            const ResSlice e = sl[q];
+            const int lg = (e.meta >> 8) & 0xf;
+            const double t = slice_sum<double, double>(e.pair0, e.meta & 0xff, lg, idx, val, xs, lane);
+            if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < (e.meta >> 12)) ys[e.pos0 + (lane >> lg)] = t / nz;
+        }
+        lost = cluster_exchange(ys + r.pos_a0, bytes_y, 8u * r.m, bar + 1, it & 1, a.cluster, rank, lost);
+        for (int q = warp; q < r.ns_t; q += W) {
+            const ResSlice e = sl[q];
+            const int lg = (e.meta >> 8) & 0xf;
+            const double t = slice_sum<double, double>(e.pair0, e.meta & 0xff, lg, idx, val, ys, lane);
+            if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < (e.meta >> 12)) xs[e.pos0 + (lane >> lg)] = t;
+        }
+    }
+    if (lost && tid == 0) atomicExch(a.error, 1);
+    if (rank == 0 && tid == 0) a.scal[static_cast<size_t>(r.inst) * a.scal_stride + a.lambda] = lambda;
+    if (a.cluster > 1) cluster_sync();
 }
 
 // ---------------------------------------------------------------- packing (device, once per plan)

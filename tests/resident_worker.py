@@ -44,6 +44,7 @@ def main(out):
                 with gb.BatchSolver(lps, opt) as bs:
                     for k, r in enumerate(bs.solve(opt)):
                         got[f"{name}.{prec}.{ce}.{k}"] = np.concatenate([[r.iterations], r.x, r.y])
+                        got[f"norm.{name}.{k}"] = np.array([r.norm_a])
     np.savez(out, **got)
 
 
