@@ -905,13 +905,13 @@ void ensure_resident(Problem& P) {
         p.cluster = C;
         int ns = 0;
         for (const ResCta& c : p.deal.cta) ns = std::max(ns, std::max(c.ns_t, c.ns_a));
-        p.threads = ns <= 8 ? 256 : (ns <= 16 || p.smem <= kResMaxSmem / 2 ? 512 : 1024);
+        p.threads = ns <= 8 ? 256 : (ns <= 16 || p.smem <= kResHalfSmem ? 512 : 1024);
         placed.push_back(std::move(p));
         R.resident[k] = 1;
     }
     if (placed.empty()) return;
     // classes: cluster size, threads and how many CTAs an SM holds; the heaviest instances first
-    auto bucket = [](const Placed& p) { return p.smem > kResMaxSmem / 2 ? 0 : p.smem > kResMaxSmem / 4 ? 1 : 2; };
+    auto bucket = [](const Placed& p) { return p.smem > kResHalfSmem ? 0 : p.smem > kResMaxSmem / 4 ? 1 : 2; };
     std::stable_sort(placed.begin(), placed.end(), [&](const Placed& x, const Placed& y) {
         if (x.cluster != y.cluster) return x.cluster > y.cluster;
         if (x.threads != y.threads) return x.threads > y.threads;
@@ -1245,11 +1245,14 @@ void build_grid(Problem& P, GridPlan& R) {
         second.raw(R.list[sd], list0[sd][kGridCtas]);
     }
     second.raw(R.idx, static_cast<size_t>(pairs) * 32);
-    second.raw(R.gx, P.n);
-    second.raw(R.gy, P.m);
-    second.raw(R.sync, 2);
+    constexpr size_t words = kGridRing * (sizeof(V) / 4);  // 64-bit words per entry of the rings
+    second.raw(R.gx, words * P.n);
+    second.raw(R.gy, words * P.m);
+    second.raw(R.sync, 3);
     second.commit(R.mem[1], P.pinned, s);
-    GB_CUDA(cudaMemsetAsync(R.sync, 0, 2 * sizeof(unsigned), s));
+    GB_CUDA(cudaMemsetAsync(R.sync, 0, 3 * sizeof(unsigned), s));
+    GB_CUDA(cudaMemsetAsync(R.gx, 0, 8 * words * P.n, s));  // tags start at 1
+    GB_CUDA(cudaMemsetAsync(R.gy, 0, 8 * words * P.m, s));
     for (int sd = 0; sd < 2; ++sd) {
         const int words = div_up(mats[sd]->cols, 32);
         k_grid_lists<<<kGridCtas, kThreads, 0, s>>>(words, R.bits[sd], R.before[sd], R.list0[sd], R.pos[1 - sd],
@@ -1298,7 +1301,7 @@ void launch_grid(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     const GridPlan& R = P.grid[sizeof(V) == 8];
     const bool odd = (ce & 1) != 0;
     GridArgs<M, V> a{R.cta, R.slices, R.idx, grid_values<M>(R), R.list[0], R.list[1],
-                     R.src[0], R.src[1], reinterpret_cast<V*>(R.gx), reinterpret_cast<V*>(R.gy),
+                     R.src[0], R.src[1], R.gx, R.gy, P.n, P.m,
                      vs.x0.get(), vs.y0.get(), odd ? vs.x1.get() : vs.x0.get(), odd ? vs.y1.get() : vs.y0.get(),
                      vs.sumx.get(), vs.sumy.get(), vs.c.get(), vs.l.get(), vs.u.get(), vs.lo.get(), vs.hi.get(),
                      P.st.get(), R.sync, P.phase_flags.get() + P.count, ce};

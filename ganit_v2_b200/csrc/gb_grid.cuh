@@ -6,16 +6,25 @@
 // 16.6 us at 2.9M in FP32.  Here every CTA owns a contiguous share of A^T's
 // rows and of A's rows (by nonzeros) with its matrix entries, vectors and
 // iterate in shared memory.  The entries of y and xbar that its rows gather --
-// for an LP with any locality a small part -- are listed once; after a grid
-// barrier the CTA copies them from L2 into shared memory and gathers there
+// for an LP with any locality a small part -- are listed once; every half
+// iteration the CTA copies them from L2 into shared memory and gathers there
 // through 16-bit local positions.  Packing, lanes per row and so the FP32 bits
 // are k_resident's; slices that do not fit the shared memory are read from L2.
 //
-// What bounds it: two barriers (~1.2 us each) and a copy from L2 after each at
-// small sizes; at 2.9M nonzeros the shared-memory wavefronts of the sums and the
-// 40 % of the matrix that comes from L2.  Measured on B200, us an iteration,
-// streaming -> here: blending 120K nonzeros FP64 9.2 -> 6.2, 411K FP64 14.6 ->
-// 7.1, 2.9M FP32 18.7 -> 13.2; random 6000 x 15001 (no locality) FP64 10.4 -> 7.3.
+// No barrier separates the halves: an entry travels with the iteration's tag
+// (FP32: value and tag in one 64-bit word, FP64: two words, each half with the
+// tag; a 64-bit access is never torn), and a reader asks again until the tag is
+// there.  A CTA thus waits for the entries it needs and no others.  Entries
+// live in rings of kGridRing slots; a grid barrier every kGridRing - 1
+// iterations keeps a writer from reaching a slot that is still read (between
+// two barriers at most kGridRing consecutive y's are alive).
+//
+// What bounds it: two trips through L2 per iteration at small sizes; at 2.9M
+// nonzeros the shared-memory wavefronts of the sums and the 40 % of the matrix
+// that comes from L2.  Measured on B200, us an iteration, streaming -> with two
+// grid barriers an iteration -> with tags: blending 120K nonzeros FP64 9.2 -> 6.2
+// -> 4.3, 411K FP64 14.6 -> 7.1 -> 5.7, 2.9M FP32 18.7 -> 13.2 -> 11.9; random
+// 6000 x 15001 (no locality) FP64 10.4 -> 7.3 -> 7.5, FP32 9.5 -> 7.2 -> 7.4.
 #pragma once
 #include "gb_qp_chip.cuh"
 #include "gb_resident.cuh"
@@ -25,7 +34,8 @@ namespace gb {
 constexpr int kGridThreads = 1024;
 constexpr int kGridCtas = 148;
 constexpr size_t kGridSmem = 226 * 1024;
-constexpr int kGridAhead = 4;  // list entries a thread reads before the barrier
+constexpr int kGridRing = 8;
+constexpr int kGridTries = 1 << 21;
 
 struct GridCta {
     int slice0, ns_t, ns_a;
@@ -53,7 +63,9 @@ struct GridArgs {
     const M* val;
     const int* list_t; const int* list_a;  // packed positions of the gathered rows / columns
     const int* col_at; const int* row_at;  // packed position -> column / row
-    V* xg; V* yg;                          // xbar and y by packed position
+    unsigned long long* xg;                // rings of xbar and y by packed position, with tags
+    unsigned long long* yg;
+    int n, m;
     const V* x0; const V* y0;
     V* x; V* y; V* sumx; V* sumy;
     const V* c; const V* l; const V* u; const V* lo; const V* hi;
@@ -63,6 +75,29 @@ struct GridArgs {
     int iters;
 };
 
+// A value and its tag to / from L2.
+__device__ __forceinline__ void put_tagged(unsigned long long* p, float v, unsigned tag) {
+    const unsigned long long w = static_cast<unsigned long long>(tag) << 32 | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ void put_tagged(unsigned long long* p, double v, unsigned tag) {
+    const unsigned long long b = __double_as_longlong(v), t = static_cast<unsigned long long>(tag) << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ bool get_tagged(const unsigned long long* p, unsigned tag, float& v) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    v = __uint_as_float(static_cast<unsigned>(w));
+    return static_cast<unsigned>(w >> 32) == tag;
+}
+__device__ __forceinline__ bool get_tagged(const unsigned long long* p, unsigned tag, double& v) {
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    v = __longlong_as_double((b << 32) | (a & 0xffffffffull));
+    return static_cast<unsigned>(a >> 32) == tag && static_cast<unsigned>(b >> 32) == tag;
+}
+
 template <class M, class V>
 __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ GridArgs<M, V> a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -71,6 +106,8 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
     const GridCta r = a.cta[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int T = kGridThreads, W = T / 32;
+    constexpr size_t kW = sizeof(V) / 4;  // words of a tagged entry
+    const unsigned base = a.sync[2];      // tags of this launch: base + 1 + iteration
     auto r4 = [](int k) { return (k + 3) & ~3; };
     V* xs = reinterpret_cast<V*>(smem);
     V* ys = xs + r4(r.u_a + 1);
@@ -107,7 +144,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
         const int i = a.row_at[r.pos_a0 + k];
         const V v = a.y0[i];
         oy[k] = v;
-        __stcg(a.yg + r.pos_a0 + k, v);
+        put_tagged(a.yg + kW * (r.pos_a0 + k), v, base + 1);
         olo[k] = a.lo[i];
         ohi[k] = a.hi[i];
         osy[k] = a.sumy[i];
@@ -120,24 +157,42 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
     cp_async_wait_all();
     bool lost = false;
     unsigned target = 0;
-    // The barrier, then the gathered entries of a vector into `to` (the list's
-    // first entries are read before the wait, whose acquire drops the L1).
-    auto collect = [&](V* to, const V* from, const int* list, int u) {
-        int at[kGridAhead];
+    // The gathered entries of a ring slot into `to`, each once its tag is there.
+    constexpr int kAhead = sizeof(V) == 4 ? 4 : 2;  // entries a thread asks for at once
+    auto collect = [&](V* to, const unsigned long long* from, const int* list, int u, unsigned tag) {
+        for (int k0 = tid; k0 < u; k0 += kAhead * T) {
+            int at[kAhead];  // -1: taken
 #pragma unroll
-        for (int i = 0; i < kGridAhead; ++i) at[i] = tid + i * T < u ? list[tid + i * T] : 0;
-        grid_barrier(a.sync, target += kGridCtas, lost);
-        V v[kGridAhead];
+            for (int i = 0; i < kAhead; ++i) at[i] = k0 + i * T < u ? list[k0 + i * T] : -1;
+            int tries = lost ? kGridTries : 0;
+            for (bool open = true; open;) {
+                V v[kAhead];
+                bool ok[kAhead];
 #pragma unroll
-        for (int i = 0; i < kGridAhead; ++i) v[i] = tid + i * T < u ? __ldcg(from + at[i]) : V(0);
+                for (int i = 0; i < kAhead; ++i) ok[i] = at[i] >= 0 && get_tagged(from + kW * at[i], tag, v[i]);
+                open = false;
 #pragma unroll
-        for (int i = 0; i < kGridAhead; ++i)
-            if (tid + i * T < u) to[tid + i * T] = v[i];
-        for (int k = tid + kGridAhead * T; k < u; k += T) to[k] = __ldcg(from + list[k]);
+                for (int i = 0; i < kAhead; ++i) {
+                    if (ok[i]) {
+                        to[k0 + i * T] = v[i];
+                        at[i] = -1;
+                    }
+                    open |= at[i] >= 0;
+                }
+                if (open && ++tries > kGridTries) {
+                    lost = true;
+                    break;
+                }
+            }
+        }
         __syncthreads();
     };
+    __syncthreads();
     for (int it = 0; it < a.iters; ++it) {
-        collect(ys, a.yg, a.list_t + r.list_t0, r.u_t);
+        const int slot = it % kGridRing;
+        const unsigned tag = base + 1 + it;
+        if (it > 0 && it % (kGridRing - 1) == 0) grid_barrier(a.sync, target += kGridCtas, lost);
+        collect(ys, a.yg + kW * slot * a.m, a.list_t + r.list_t0, r.u_t, tag);
         for (int q = warp; q < r.ns_t; q += W) {  // primal half (PrimalEpi)
             const ResSlice e = sl[q];
             const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
@@ -153,10 +208,11 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
             if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < nr) {
                 ox[k] = v;
                 osx[k] = sk + v;
-                __stcg(a.xg + r.pos_t0 + k, V(2) * v - xk);
+                put_tagged(a.xg + kW * (static_cast<size_t>(slot) * a.n + r.pos_t0 + k), V(2) * v - xk, tag);
             }
         }
-        collect(xs, a.xg, a.list_a + r.list_a0, r.u_a);
+        collect(xs, a.xg + kW * slot * a.n, a.list_a + r.list_a0, r.u_a, tag);
+        const size_t next = static_cast<size_t>((it + 1) % kGridRing) * a.m;
         for (int q = warp; q < r.ns_a; q += W) {  // dual half (DualEpi)
             const ResSlice e = sl[r.ns_t + q];
             const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
@@ -173,7 +229,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
             if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < nr) {
                 osy[k] = sk + v;
                 oy[k] = v;
-                __stcg(a.yg + r.pos_a0 + k, v);
+                put_tagged(a.yg + kW * (next + r.pos_a0 + k), v, tag + 1);
             }
         }
     }
@@ -188,6 +244,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
         a.y[i] = oy[k];
         a.sumy[i] = osy[k];
     }
+    lost = __syncthreads_or(lost);
     if (tid == 0) {
         if (lost) {  // the solve stops at the coming check and reports the error
             atomicExch(a.error, 1);
@@ -197,6 +254,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ G
         if (atomicAdd(a.sync + 1, 1u) == kGridCtas - 1) {  // every CTA has passed its last barrier
             a.sync[0] = 0u;
             a.sync[1] = 0u;
+            a.sync[2] = base + static_cast<unsigned>(a.iters) + 1u;
         }
     }
 }
@@ -295,7 +353,7 @@ struct GridPlan {
     unsigned char* lg[2] = {};
     long long* pair0[2] = {};
     unsigned* idx = nullptr;
-    double *gx = nullptr, *gy = nullptr;           // xbar / y by packed position
+    unsigned long long *gx = nullptr, *gy = nullptr;  // rings of xbar / y by packed position
     unsigned* sync = nullptr;
     DevBuf<float> val32;
     DevBuf<double> val64;

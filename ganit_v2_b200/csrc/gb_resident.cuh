@@ -45,6 +45,7 @@ constexpr int kResMaxSteps = 32;                       // lane steps of a row (k
 constexpr int kResBins = kResMaxSteps / 2 + 1;         // step pairs 0..16
 constexpr int kResMaxIndex = 65535;                    // positions are 16 bits wide
 constexpr size_t kResMaxSmem = 227 * 1024;             // shared memory of one CTA
+constexpr size_t kResHalfSmem = 113 * 1024;           // of two CTAs on an SM (1 KB each is reserved)
 constexpr int kResMaxCluster = 16;
 constexpr int kResLaneSteps64 = 8;                     // FP64: lanes per row so that a lane adds at most this many
 
