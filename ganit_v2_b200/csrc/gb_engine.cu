@@ -274,9 +274,9 @@ void init_kernel_attrs() {
         set_smem(k_grid<__nv_bfloat16, float>, kGridSmem);
         set_smem(k_grid<float, double>, kGridSmem);
         set_smem(k_grid<double, double>, kGridSmem);
-        set_smem(k_qp_chip<float, float>, kQpSmem);
-        set_smem(k_qp_chip<float, double>, kQpSmem);
-        set_smem(k_qp_chip<double, double>, kQpSmem);
+        set_smem(k_qp_chip<float, float>, kQpSmem<float>);
+        set_smem(k_qp_chip<float, double>, kQpSmem<double>);
+        set_smem(k_qp_chip<double, double>, kQpSmem<double>);
     });
 }
 
@@ -1022,24 +1022,25 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     a.at_val = P.AT.val<M>();
     a.at_lg = sizeof(V) == 4 ? P.qp_at_lg.get() : nullptr;
     a.A = P.A.view<M>();
-    a.slots = P.qp_slots.get();
+    a.slots = P.qp_words.get();
+    a.xbar = a.slots + 4 * kQpMaxSlots;
+    a.t = a.xbar + ((P.n + 1) & ~1);  // 16-byte words
+    a.part = a.t + 2 * (kMaxRank + kQpMaxRows);
     const std::vector<RowBlock>& blocks = P.A.template sched_for<M>().host_blocks;
     for (int b = 0; b < a.A.nb; ++b)
         for (int r = blocks[b].r0; r < blocks[b].r1; ++r) {
             if (blocks[b].kind == kStream) a.slot0[r] = a.A.nb + r;
             else if (a.nslots[r] == 0) a.slot0[r] = b;
-            ++a.nslots[r];
+            const int z = a.slot0[r] + a.nslots[r]++;
+            a.used[z >> 6] |= 1ull << (z & 63);
         }
     a.total_slots = a.A.nb + P.m;
     a.x0 = vs.x0.get();
     a.y0 = vs.y0.get();
     a.x = odd ? vs.x1.get() : vs.x0.get();
     a.y = odd ? vs.y1.get() : vs.y0.get();
-    a.xbar = vs.xbar.get();
     a.sumx = vs.sumx.get();
     a.sumy = vs.sumy.get();
-    a.part = P.partials.get();
-    a.t = P.ftx.get();
     a.st = a.st_rw = P.st.get();
     a.sync = P.qp_sync.get();
     a.error = P.phase_flags.get() + P.count;
@@ -1047,7 +1048,7 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(kQpGrid);
     cfg.blockDim = dim3(kQpThreads);
-    cfg.dynamicSmemBytes = kQpSmem;
+    cfg.dynamicSmemBytes = kQpSmem<V>;
     cfg.stream = s;
     attr[0].id = cudaLaunchAttributeCooperative;  // its CTAs wait for one another
     attr[0].val.cooperative = 1;
@@ -1328,8 +1329,9 @@ void prepare_resident(Problem& P) {
     if (P.dplr && !P.qp_sync.get()) {
         P.qp_sync.reset(2);
         GB_CUDA(cudaMemsetAsync(P.qp_sync.get(), 0, 2 * sizeof(unsigned), P.stream));
-        P.qp_slots.reset(kQpMaxSlots);
-        GB_CUDA(cudaMemsetAsync(P.qp_slots.get(), 0, kQpMaxSlots * sizeof(double), P.stream));
+        P.qp_words.reset(4 * kQpMaxSlots + P.n + 1 + 2 * (kMaxRank + kQpMaxRows) +
+                         2 * static_cast<size_t>(kMaxRank + kQpMaxRows) * kFtxGrid);
+        GB_CUDA(cudaMemsetAsync(P.qp_words.get(), 0, P.qp_words.size() * 8, P.stream));  // tags start at 1
     }
     if (P.dplr && sizeof(V) == 4 && !P.qp_at_lg.get() && qp_on_chip<float, V>(P)) {
         const DevSchedule& st = P.AT.template sched_for<V>();

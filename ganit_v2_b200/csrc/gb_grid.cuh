@@ -75,29 +75,6 @@ struct GridArgs {
     int iters;
 };
 
-// A value and its tag to / from L2.
-__device__ __forceinline__ void put_tagged(unsigned long long* p, float v, unsigned tag) {
-    const unsigned long long w = static_cast<unsigned long long>(tag) << 32 | __float_as_uint(v);
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
-}
-__device__ __forceinline__ void put_tagged(unsigned long long* p, double v, unsigned tag) {
-    const unsigned long long b = __double_as_longlong(v), t = static_cast<unsigned long long>(tag) << 32;
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
-                 : "memory");
-}
-__device__ __forceinline__ bool get_tagged(const unsigned long long* p, unsigned tag, float& v) {
-    unsigned long long w;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
-    v = __uint_as_float(static_cast<unsigned>(w));
-    return static_cast<unsigned>(w >> 32) == tag;
-}
-__device__ __forceinline__ bool get_tagged(const unsigned long long* p, unsigned tag, double& v) {
-    unsigned long long a, b;
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-    v = __longlong_as_double((b << 32) | (a & 0xffffffffull));
-    return static_cast<unsigned>(a >> 32) == tag && static_cast<unsigned>(b >> 32) == tag;
-}
-
 template <class M, class V>
 __global__ void __launch_bounds__(kGridThreads) k_grid(const __grid_constant__ GridArgs<M, V> a) {
     extern __shared__ __align__(16) unsigned char smem[];

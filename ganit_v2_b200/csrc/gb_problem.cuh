@@ -150,8 +150,8 @@ struct Problem {
     DevBuf<RowBlock> list_a, list_t;
     int list_na = 0, list_nt = 0, list_level = -1;
     DevBuf<unsigned char> qp_at_lg;       // k_qp_chip: log2 lanes per row of A^T (FP32)
-    DevBuf<unsigned> qp_sync;             // k_qp_chip's {arrivals, exits}
-    DevBuf<double> qp_slots;              // and its row sums
+    DevBuf<unsigned> qp_sync;             // k_qp_chip's {exits, tag base}
+    DevBuf<unsigned long long> qp_words;  // and its tagged exchange
     GridPlan grid[2];                     // a single LP kept by the whole GPU: FP32 vectors, FP64 vectors
     ResPlan res[2];                       // instances iterated on chip: FP32 vectors, FP64 vectors
     double setup_seconds = 0.0;
