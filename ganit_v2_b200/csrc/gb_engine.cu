@@ -791,14 +791,14 @@ void launch_resident(Problem& P, VecSet<V>& vs, const ResClass& c, int ce, cudaS
 // Packed values of one type (made on first use; the structure is there).
 template <class Buf, class Src>
 void pack_values(Problem& P, Buf& buf, long long pairs, const int* slot_t, const int* slot_a, const ResSliceAt* at,
-                 Src src) {
+                 const unsigned char* step_t, const unsigned char* step_a, Src src) {
     if (buf.get()) return;
     cudaStream_t s = P.stream;
     buf.reset(static_cast<size_t>(pairs) * 64);
     GB_CUDA(cudaMemsetAsync(buf.get(), 0, buf.size() * sizeof(*buf.get()), s));
     const int gt = elem_grid(P.n, P.sms), ga = elem_grid(P.m, P.sms);
-    k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), slot_t, at, buf.get());
-    k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), slot_a, at, buf.get());
+    k_res_values<<<gt, kThreads, 0, s>>>(P.n, P.AT.ptr.get(), src(P.AT), slot_t, at, step_t, buf.get());
+    k_res_values<<<ga, kThreads, 0, s>>>(P.m, P.A.ptr.get(), src(P.A), slot_a, at, step_a, buf.get());
     GB_CUDA(cudaGetLastError());
 }
 
@@ -806,7 +806,7 @@ template <class M, class V>
 void ensure_resident_values(Problem& P) {
     ResPlan& R = P.res[sizeof(V) == 8];
     if (!R.any()) return;
-    auto pack = [&](auto& buf, auto src) { pack_values(P, buf, R.pairs, R.slot_t, R.slot_a, R.at, src); };
+    auto pack = [&](auto& buf, auto src) { pack_values(P, buf, R.pairs, R.slot_t, R.slot_a, R.at, R.step_t, R.step_a, src); };
     if constexpr (std::is_same<M, double>::value) pack(R.val64, [](const DevMat& A) { return A.val64.get(); });
     else if constexpr (std::is_same<M, float>::value) pack(R.val32, [](const DevMat& A) { return A.val32.get(); });
     else pack(R.valbf, [](const DevMat& A) { return A.valbf.get(); });
@@ -963,6 +963,9 @@ void ensure_resident(Problem& P) {
     if (w == 0) {
         arena.raw(R.lg_t, P.n);
         arena.raw(R.lg_a, P.m);
+    } else {
+        arena.raw(R.step_t, P.A.nnz);
+        arena.raw(R.step_a, P.A.nnz);
     }
     arena.commit(R.mem, P.pinned, s);
     if (w == 0) {
@@ -974,10 +977,16 @@ void ensure_resident(Problem& P) {
     k_res_rank<<<ns, 32, 0, s>>>(R.sides_a, P.A.ptr.get(), R.lg_a, R.at, R.slot_a, R.pos_a, R.row_at);
     k_res_fill<<<static_cast<int>(T.cta.size()), kThreads, 0, s>>>(R.cta, R.idx);
     unsigned short* idx16 = reinterpret_cast<unsigned short*>(R.idx);
+    if (w) {
+        ResOrderArgs o{{{R.col_at, P.AT.ptr.get(), P.AT.idx.get(), R.pos_a, R.step_t},
+                        {R.row_at, P.A.ptr.get(), P.A.idx.get(), R.pos_t, R.step_a}}};
+        const int ns = static_cast<int>(T.at.size());
+        k_res_order<<<div_up(ns, 4), 128, 0, s>>>(ns, R.at, o);
+    }
     k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t, R.at,
-                                                             R.pos_a, idx16);
+                                                             R.pos_a, R.step_t, idx16);
     k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a, R.at,
-                                                             R.pos_t, idx16);
+                                                             R.pos_t, R.step_a, idx16);
     GB_CUDA(cudaGetLastError());
     if (trace_enabled())
         for (const ResClass& c : R.classes)
@@ -1292,9 +1301,9 @@ template <class M, class V>
 void ensure_grid_values(Problem& P) {
     GridPlan& R = P.grid[sizeof(V) == 8];
     if (!R.on) return;
-    if constexpr (std::is_same<M, double>::value) pack_values(P, R.val64, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.val64.get(); });
-    else if constexpr (std::is_same<M, float>::value) pack_values(P, R.val32, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.val32.get(); });
-    else pack_values(P, R.valbf, R.pairs, R.slot[0], R.slot[1], R.at, [](const DevMat& A) { return A.valbf.get(); });
+    if constexpr (std::is_same<M, double>::value) pack_values(P, R.val64, R.pairs, R.slot[0], R.slot[1], R.at, nullptr, nullptr, [](const DevMat& A) { return A.val64.get(); });
+    else if constexpr (std::is_same<M, float>::value) pack_values(P, R.val32, R.pairs, R.slot[0], R.slot[1], R.at, nullptr, nullptr, [](const DevMat& A) { return A.val32.get(); });
+    else pack_values(P, R.valbf, R.pairs, R.slot[0], R.slot[1], R.at, nullptr, nullptr, [](const DevMat& A) { return A.valbf.get(); });
 }
 
 template <class M, class V>
