@@ -651,6 +651,7 @@ EvalArgs<M, V> eval_args(Problem& P, VecSet<V>& vs, const V* x, const V* y, int 
     a.qxa = (with_q && mode == kEvalCheck) ? vs.qxa.get() : nullptr;
     a.mode = mode;
     a.count = P.count;
+    a.per_cta = decide_inst(P.count);
     a.seg_a = P.A.sched_for<M>().seg_block.get();
     a.seg_t = P.AT.sched_for<M>().seg_block.get();
     a.st = P.st.get();

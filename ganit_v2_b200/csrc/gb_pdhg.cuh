@@ -252,14 +252,18 @@ struct EvalArgs {
     unsigned long long cond;     // cudaGraphConditionalHandle of the phase loop
     int use_cond;                // 1 inside the loop body: the decision drives the loop
     unsigned* sync = nullptr;    // k_decide over several CTAs: {arrivals, any instance active}
+    int per_cta = 1;             // k_decide: decide_inst(count)
     int terms_ready = 0;         // single instance: k_terms summed its terms into inst_terms
 };
 
-// k_decide's grid: one CTA for a single problem, else one CTA per
-// kDecideInst instances (one instance per warp while reducing).
-constexpr int kDecideInst = kWarps;
+// Instances per CTA of k_decide: one up to 256 instances (a CTA per instance
+// folds and decides in ~8 us where eight took 13-18: 37 LPs 2.77 -> 2.65 ms, 64
+// branching children 152 -> 148.5), up to kDecideInst in larger batches, whose
+// CTAs would queue (no difference at 512).
+constexpr int kDecideInst = 8;
+inline int decide_inst(int count) { return std::min(kDecideInst, std::max(1, count / 256)); }
 constexpr int kDecideWide = 128;  // blocks above which an instance's terms are summed by a whole CTA
-inline int decide_grid(int count) { return count == 1 ? 1 : (count + kDecideInst - 1) / kDecideInst; }
+inline int decide_grid(int count) { return (count + decide_inst(count) - 1) / decide_inst(count); }
 
 template <class V>
 __device__ __forceinline__ V avg_of(const V* s, int k, double inv) {
@@ -548,9 +552,9 @@ __global__ void __launch_bounds__(kThreads) k_eval(const __grid_constant__ EvalA
 
 // After k_eval: reduce every instance's partials in a fixed order and run its
 // decision.  A single problem is one CTA; a batch gets one CTA per
-// kDecideInst instances (decide_grid).  Within a CTA an instance with many
-// blocks is reduced by the whole CTA (one at a time); the others by one warp
-// each into inst_terms, after which every thread runs the decisions of its own
+// decide_inst(count) instances.  Within a CTA an instance with many
+// blocks is reduced by the whole CTA (one at a time); the others term by term
+// over the warps into inst_terms, after which every thread runs the decisions of its own
 // instances (the scalar decision code is the long part, so it must not run one
 // instance per warp).  With several CTAs the last to arrive sets the phase
 // loop's condition from the OR of every CTA's "some instance still active" and
@@ -580,8 +584,8 @@ __global__ void __launch_bounds__(kThreads) k_decide(const __grid_constant__ Eva
     __shared__ double red[kWarps * kTerms];
     const int nbA = a.A.nb;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int k0 = gridDim.x == 1 ? 0 : blockIdx.x * kDecideInst;
-    const int k1 = gridDim.x == 1 ? a.count : min(a.count, k0 + kDecideInst);
+    const int k0 = gridDim.x == 1 ? 0 : blockIdx.x * a.per_cta;
+    const int k1 = gridDim.x == 1 ? a.count : min(a.count, k0 + a.per_cta);
     int any_active = 0;
     auto load_terms = [&](int k, int first, int step, double (&T)[kTerms]) {
 #pragma unroll
