@@ -859,24 +859,32 @@ void ensure_resident(Problem& P) {
         total += wk;
     }
     if (who.empty()) return;
-    // the largest cluster that this GPU can place with the largest shared memory
-    static std::array<std::atomic<int>, 2> most_cluster{};
-    if (most_cluster[w].load() == 0) {
-        int best = 8;
+    // how many clusters of each size this GPU holds at once with the largest
+    // shared memory (a GPC's SMs are not a multiple of 16: 7 of 16, not 9)
+    static std::array<std::array<std::atomic<int>, 5>, 2> fits{};
+    std::array<int, 5> active{};
+    for (int l = 0; l < 5; ++l) {
+        active[l] = fits[w][l].load();
+        if (active[l] > 0) continue;
         ResClass c;
-        c.cluster = kResMaxCluster;
+        c.cluster = 1 << l;
         c.threads = 512;
-        c.nctas = kResMaxCluster;
+        c.nctas = c.cluster;
         c.smem = kResMaxSmem;
         cudaLaunchAttribute attr[1];
         const cudaLaunchConfig_t cfg = resident_config(c, attr, P.stream);
         int got = 0;
-        if (cudaOccupancyMaxActiveClusters(&got, resident_kernel<V, V>(512), &cfg) == cudaSuccess && got > 0)
-            best = kResMaxCluster;
+        if (cudaOccupancyMaxActiveClusters(&got, resident_kernel<V, V>(512), &cfg) != cudaSuccess) got = 0;
         cudaGetLastError();
-        most_cluster[w].store(best);
+        active[l] = got > 0 ? got : -1;
+        fits[w][l].store(active[l]);
     }
-    const int cmax = most_cluster[w].load();
+    auto log2_of = [](int c) {
+        int l = 0;
+        while (c >>= 1) ++l;
+        return l;
+    };
+    const int cmax = active[4] > 0 ? kResMaxCluster : 8;
     struct Placed {
         int k, at;
         ResDeal deal;
@@ -893,16 +901,25 @@ void ensure_resident(Problem& P) {
         while (2 * C <= cmax && 2 * C <= share && slices >= 2 * C * kResMinSlices) C *= 2;
         Placed p{k, static_cast<int>(q), {}, work[q], 0, 0, 0};
         const std::array<ResHist, 2>& HH = hist[q];
-        for (; C <= cmax; C *= 2) {
+        auto deal = [&](int c, Placed& to) {
             const long long pairs = HH[0].pairs + HH[1].pairs;
-            if (static_cast<size_t>(pairs) * (128 + 64 * sm) > C * kResMaxSmem) continue;  // cannot fit
-            res_deal(HH, C, p.deal);
-            p.smem = p.deal.smem(sm, sizeof(V));
+            if (static_cast<size_t>(pairs) * (128 + 64 * sm) > c * kResMaxSmem) return false;  // cannot fit
+            res_deal(HH, c, to.deal);
+            to.smem = to.deal.smem(sm, sizeof(V));
             if (w)
-                for (const ResCta& c : p.deal.cta) p.smem = std::max(p.smem, power_smem_bytes(c));
-            if (p.smem <= kResMaxSmem) break;
-        }
+                for (const ResCta& cta : to.deal.cta) to.smem = std::max(to.smem, power_smem_bytes(cta));
+            return to.smem <= kResMaxSmem;
+        };
+        while (C <= cmax && !deal(C, p)) C *= 2;
         if (C > cmax) continue;
+        // One CTA per SM, and shares of this size need a second wave: half the
+        // cluster if that holds it.  16 x (5000 x 200) in FP64: 7.8 us an
+        // iteration in clusters of 8 (15 at once), 5.1 in clusters of 4.
+        for (; C > 1 && p.smem > kResHalfSmem && share * active[log2_of(C)] < P.sms; C /= 2) {
+            Placed half{k, static_cast<int>(q), {}, work[q], 0, 0, 0};
+            if (!deal(C / 2, half)) break;
+            p = std::move(half);
+        }
         p.cluster = C;
         int ns = 0;
         for (const ResCta& c : p.deal.cta) ns = std::max(ns, std::max(c.ns_t, c.ns_a));
@@ -910,6 +927,30 @@ void ensure_resident(Problem& P) {
         placed.push_back(std::move(p));
         R.resident[k] = 1;
     }
+    // Clusters in waves (one CTA per SM): a wave takes 4.7-7.5 us an iteration,
+    // in which the streaming kernels read about 16 MB of such a batch from L2.
+    // So instances that need the largest cluster, which leaves a quarter of the
+    // SMs idle, stream when they do not fit one wave, and smaller ones in more
+    // than two waves stream when a wave of them has less than that to read.
+    // us an iteration, on chip / streaming: 64 x (20000 x 500, 100K nonzeros)
+    // FP32 71 / 54 and 64 x (10000 x 500, 50K) FP64 62 / 39 in clusters of 16,
+    // but 4 of them 7.7 / 14.0 and 6.8 / 11.4; 64 x (7500 x 200, 15K) FP64 (14
+    // MB a wave) 24 / 18 in clusters of 8, but 64 x (6500 x 400, 31K) FP64 (19
+    // MB) 25 / 26 and 64 x (10000 x 500) FP32 (18 MB) 24 / 28.
+    constexpr double kWaveBytes = 16e6;
+    std::array<int, 5> clusters{};
+    for (const Placed& p : placed)
+        if (p.smem > kResHalfSmem) ++clusters[log2_of(p.cluster)];
+    auto streams = [&](const Placed& p) {
+        const int l = log2_of(p.cluster);
+        if (p.smem <= kResHalfSmem || clusters[l] <= active[l] * (p.cluster == cmax ? 1 : 2)) return false;
+        const double nnz = P.nnz_off[p.k + 1] - P.nnz_off[p.k], n = P.col_off[p.k + 1] - P.col_off[p.k],
+                     m = P.row_off[p.k + 1] - P.row_off[p.k];
+        return p.cluster == cmax || active[l] * (2.0 * (4 + sm) * nnz + sm * (9.0 * n + 7.0 * m)) < kWaveBytes;
+    };
+    for (const Placed& p : placed)
+        if (streams(p)) R.resident[p.k] = 0;
+    placed.erase(std::remove_if(placed.begin(), placed.end(), streams), placed.end());
     if (placed.empty()) return;
     // classes: cluster size, threads and how many CTAs an SM holds; the heaviest instances first
     auto bucket = [](const Placed& p) { return p.smem > kResHalfSmem ? 0 : p.smem > kResMaxSmem / 4 ? 1 : 2; };
