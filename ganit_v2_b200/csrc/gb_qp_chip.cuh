@@ -26,11 +26,17 @@
 // 100,000 x 50 F is 40 MB, the SMs' shared memories hold ~31) come from L2: read
 // early, one warp per row, and summed by shuffles.
 //
-// What bounds it (100,000 x 50, FP64, 22 K cycles an iteration): the two reads
-// of F from shared memory and their FP64 chains (13 K), two barriers (5.5 K).
-// Measured on B200, start -> now: 100,000 x 50 FP64 29 -> 12.7 us an iteration,
-// 8,009 x 33 mixed 18.5 -> 7.0 us.  With the chunks' last arrival running the
-// dual step, and x and bounds read behind the barrier, it was 16 and 10 us.
+// What bounds it (100,000 x 50, FP64, ~20 K cycles an iteration): the two reads
+// of F from shared memory and their FP64 chains (13 K), then three trips of the
+// words through L2.  8,009 x 33 is the trips alone: 9 % of the shared-memory
+// wavefronts, warps waiting for words.
+// Measured on B200, streaming -> here: 100,000 x 50 FP64 29 -> 11.7 us an
+// iteration, 8,009 x 33 mixed 18.5 -> 6.0 us.  With two grid barriers an
+// iteration in place of the tags it was 12.7 and 7.0 us; with the last arrival
+// of a chunk running the dual step, and x and bounds read behind the barrier,
+// 16 and 10 us.  Reading F once (a warp per four columns, partials by
+// transposing shuffles) took 20.4 and 7.0 us against 14.5 and 8.1 at that
+// point: the shuffles cost more than the second read saves.
 #pragma once
 #include "gb_qp.cuh"
 #include "gb_resident.cuh"
