@@ -1137,6 +1137,11 @@ void build_grid(Problem& P, GridPlan& R) {
     if (P.count != 1 || P.has_q || P.res[w].any() || P.sms < kGridCtas || !resident_enabled() ||
         std::max(P.n, P.m) > kMaxVector || P.A.nnz < 1)
         return;
+    // Fewer than four rows of either side per CTA: the FP32 streaming kernels are as
+    // fast or faster.  us an iteration, here / streaming, 40000 columns x 500 rows
+    // FP32 10.4 / 8.4, x 1000 rows 8.5 / 8.5, 30000 x 3000 9.6 / 13.5; FP64 with 500
+    // rows 8.5 / 12.2.
+    if (w == 0 && std::min(P.n, P.m) < 4 * kGridCtas) return;
     // before any work: the vectors and half of the matrix against the GPU's shared memory
     const double room = static_cast<double>(kGridCtas) * kGridSmem - sizeof(V) * (5.0 * P.n + 4.0 * P.m);
     if (static_cast<double>(P.A.nnz) / 32.0 * static_cast<double>(pair_bytes) > 2.0 * room) return;
@@ -1280,7 +1285,11 @@ void build_grid(Problem& P, GridPlan& R) {
         }
         R.smem = std::max(R.smem, fixed + pair_bytes * (k.pairs_t + k.pairs_a));
     }
-    if (2 * kept < pairs) return;
+    // A matrix kept in part pays only if its rows gather less than they hold: us an
+    // iteration, here / streaming, FP64: blending 1.6M nonzeros, 62 % kept, 0.4M
+    // gathered 11.2 / 16.5; random 2000 x 60000, 71 % of 1.2M kept, 1.4M gathered
+    // 19.7 / 17.8; 20000 x 30000, 92 % of 0.9M kept, 1.6M gathered 15.4 / 14.2.
+    if (2 * kept < pairs || (kept < pairs && static_cast<long long>(list0[0][kGridCtas]) + list0[1][kGridCtas] > P.A.nnz)) return;
     R.pairs = pairs;
     std::vector<long long> p0[2];
     for (int sd = 0; sd < 2; ++sd) {
