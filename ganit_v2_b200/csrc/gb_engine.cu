@@ -178,7 +178,7 @@ void prepare_power(Problem& P);
 void launch_power_chip(Problem& P, cudaStream_t s);
 bool all_resident(const Problem& P) {
     const ResPlan& R = P.res[1];
-    return R.any() && R.list_na == 0;
+    return R.any() && R.list_na[1] == 0;
 }
 void power_iteration(Problem& P, bool q, cudaStream_t s) {
     const int n = P.n;
@@ -671,9 +671,10 @@ struct StreamBlocks {
 };
 template <class M, class V>
 StreamBlocks stream_blocks(const Problem& P) {
+    constexpr int mw = sizeof(M) == 8;
     const ResPlan& R = P.res[sizeof(V) == 8];
     if (P.list_level == level_index<M, V>()) return {P.list_a.get(), P.list_t.get(), P.list_na, P.list_nt};
-    if (R.any()) return {R.list_a, R.list_t, R.list_na, R.list_nt};
+    if (R.any()) return {R.list_a[mw], R.list_t[mw], R.list_na[mw], R.list_nt[mw]};
     return {};
 }
 
@@ -979,22 +980,22 @@ void ensure_resident(Problem& P) {
     }
     R.pairs = T.pairs;
     cudaStream_t s = P.stream;
-    std::vector<RowBlock> la, lt;
-    for (int k = 0; k < P.count; ++k) {
-        if (R.resident[k]) continue;
-        la.insert(la.end(), sa.host_blocks.begin() + sa.host_seg_block[k], sa.host_blocks.begin() + sa.host_seg_block[k + 1]);
-        lt.insert(lt.end(), st.host_blocks.begin() + st.host_seg_block[k], st.host_blocks.begin() + st.host_seg_block[k + 1]);
-    }
-    R.list_na = static_cast<int>(la.size());
-    R.list_nt = static_cast<int>(lt.size());
+    // by matrix type: FP64 vectors meet either (the FP32 matrix in Dynamic solves)
+    std::vector<RowBlock> la[2], lt[2];
+    streamed_blocks<float, V>(P, la[0], lt[0]);
+    if (w) streamed_blocks<double, V>(P, la[1], lt[1]);
     PlanArena arena;
     arena.host(R.cta, T.cta);
     arena.host(R.slices, T.slices);
     arena.host(R.at, T.at);
     arena.host(R.sides_t, T.sides[0]);
     arena.host(R.sides_a, T.sides[1]);
-    arena.host(R.list_a, la);
-    arena.host(R.list_t, lt);
+    for (int mw = 0; mw <= w; ++mw) {
+        R.list_na[mw] = static_cast<int>(la[mw].size());
+        R.list_nt[mw] = static_cast<int>(lt[mw].size());
+        arena.host(R.list_a[mw], la[mw]);
+        arena.host(R.list_t[mw], lt[mw]);
+    }
     arena.ones(R.col_at, T.positions[0]);
     arena.ones(R.row_at, T.positions[1]);
     arena.ones(R.slot_t, P.n);
@@ -1688,16 +1689,13 @@ void set_phase_lists(Problem& P) {
     if (P.count <= 1 || !phase_lists_enabled()) return;
     const DevSchedule& sa = P.A.template sched_for<M>();
     const DevSchedule& st = P.AT.template sched_for<M>();
+    constexpr int mw = sizeof(M) == 8;
     std::vector<RowBlock> la, lt;
     int part = 0;
     const ResPlan& R = P.res[sizeof(V) == 8];
-    for (int k = 0; k < P.count; ++k) {
-        part += P.phase_flags_host[k];
-        if (!P.phase_flags_host[k] || R.resident[k]) continue;
-        for (int b = sa.host_seg_block[k]; b < sa.host_seg_block[k + 1]; ++b) la.push_back(sa.host_blocks[b]);
-        for (int b = st.host_seg_block[k]; b < st.host_seg_block[k + 1]; ++b) lt.push_back(st.host_blocks[b]);
-    }
-    const size_t all = R.any() ? R.list_na + R.list_nt : sa.nb + st.nb;
+    for (int k = 0; k < P.count; ++k) part += P.phase_flags_host[k];
+    collect_blocks<M>(P, [&](int k) { return P.phase_flags_host[k] && !R.resident[k]; }, la, lt);
+    const size_t all = R.any() ? R.list_na[mw] + R.list_nt[mw] : sa.nb + st.nb;
     if (2 * (la.size() + lt.size()) > all || part == P.count) return;
     auto put = [&](DevBuf<RowBlock>& d, const std::vector<RowBlock>& h) {
         if (d.size() < h.size()) d.reset(h.size());  // a buffer only grows: graphs keep their pointer

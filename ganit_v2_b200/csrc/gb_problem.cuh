@@ -207,4 +207,24 @@ int guarded(F&& f) {
     }
 }
 
+// Row blocks of A and of A^T of the instances that `pick` takes, as the
+// kernels of matrix type M run them: cut for the schedule of their view
+// (DevMat::view), whose bitmaps, slots and counters they index.
+template <class M, class Pick>
+void collect_blocks(const Problem& P, Pick&& pick, std::vector<RowBlock>& la, std::vector<RowBlock>& lt) {
+    const DevSchedule& sa = P.A.template sched_for<M>();
+    const DevSchedule& st = P.AT.template sched_for<M>();
+    for (int k = 0; k < P.count; ++k) {
+        if (!pick(k)) continue;
+        la.insert(la.end(), sa.host_blocks.begin() + sa.host_seg_block[k], sa.host_blocks.begin() + sa.host_seg_block[k + 1]);
+        lt.insert(lt.end(), st.host_blocks.begin() + st.host_seg_block[k], st.host_blocks.begin() + st.host_seg_block[k + 1]);
+    }
+}
+// Those of the instances that stream at level <M, V>.
+template <class M, class V>
+void streamed_blocks(const Problem& P, std::vector<RowBlock>& la, std::vector<RowBlock>& lt) {
+    const ResPlan& R = P.res[sizeof(V) == 8];
+    collect_blocks<M>(P, [&](int k) { return !R.resident[k]; }, la, lt);
+}
+
 }  // namespace gb

@@ -868,9 +868,11 @@ struct ResPlan {
     DevBuf<__nv_bfloat16> valbf;
     long long pairs = 0;
     // Row blocks of the other instances, which the streaming kernels run
-    // (nothing: every instance is resident).
-    RowBlock *list_a = nullptr, *list_t = nullptr;
-    int list_na = 0, list_nt = 0;
+    // (nothing: every instance is resident), by matrix type (0: FP32 / BF16,
+    // 1: FP64): a block's bitmap, slots and counter are those of the schedule
+    // it was cut for, and the two types' schedules part when they are tuned.
+    RowBlock *list_a[2] = {}, *list_t[2] = {};
+    int list_na[2] = {}, list_nt[2] = {};
     bool any() const { return !classes.empty(); }
 };
 
