@@ -13,9 +13,11 @@
 //     a gather is a shared-memory read.  After each half iteration a CTA sends
 //     its share to every other one with a bulk copy between shared memories,
 //     which counts its bytes on the receiver's mbarrier; the receiver starts
-//     its next half when all shares are in.  A share of iteration k + 1
-//     cannot overtake one of iteration k: it depends on the receiver's own
-//     share of the half in between, sent after its last read.
+//     its next half when all shares are in.  A CTA that owns nothing on a side
+//     (few rows, many columns) arrives on the peers' mbarriers instead.  So a
+//     share of iteration k + 1 cannot overtake one of iteration k: it depends
+//     on the receiver's own share or arrival of the half in between, sent after
+//     its last read and after all of its shares of iteration k were in.
 //
 // Layout ("slices").  Rows are reduced by groups of G = 2^lg lanes, lane g of
 // a group adding entries g, g + G, ... of its row in order, then the groups'
@@ -59,6 +61,7 @@ struct ResCta {
     int n, m;                 // positions of the instance's columns / rows; entries n and m are the zero slots
     int at_t0, at_a0;         // the instance's first entries of col_at / row_at
     int pairs_t;              // A^T's step pairs, stored before A's
+    int idle_t, idle_a;       // CTAs of the cluster that own no columns / no rows
     long long pair0;          // first step pair in the packed arrays
 };
 
@@ -109,10 +112,18 @@ __device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
     return r;
 }
 
-// mbarriers of one arrival (the CTA's own) plus the bytes announced with it.
-__device__ __forceinline__ void mbar_init(unsigned long long* b) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b)))
+// Arrivals that end a phase of a vector's mbarrier, next to the bytes announced
+// with the CTA's own: that one, and one of every other CTA that owns none of
+// the vector (`idle` of the cluster; `own`: this CTA's entries).
+__host__ __device__ inline int exchange_arrivals(int idle, int own) { return 1 + idle - (own == 0 ? 1 : 0); }
+__device__ __forceinline__ void mbar_init(unsigned long long* b, int arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b))),
+                 "r"(arrivals)
                  : "memory");
+}
+// Arrival on the same mbarrier of CTA `rank`.
+__device__ __forceinline__ void mbar_arrive_peer(unsigned long long* b, int rank) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(b, rank)) : "memory");
 }
 __device__ __forceinline__ void mbar_init_visible() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect(unsigned long long* b, unsigned bytes) {
@@ -149,10 +160,11 @@ __device__ __forceinline__ void copy_to_peer(const void* p, unsigned bytes, unsi
 // Shared-memory writes of this thread, before a bulk copy reads them.
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// End of a half iteration: this CTA's share `p` of a gathered vector goes to
-// every other CTA of the cluster, and theirs are awaited (`total`: the vector's
-// bytes; `bar`: its mbarrier, at the phase of `parity`).  Returns `lost`, or
-// whether the wait ran out; once lost, later waits are skipped.
+// End of a half iteration: this CTA's share `p` of a gathered vector (or an
+// arrival, if it has none) goes to every other CTA of the cluster, and theirs
+// are awaited (`total`: the vector's bytes; `bar`: its mbarrier, at the phase
+// of `parity`).  Returns `lost`, or whether the wait ran out; once lost, later
+// waits are skipped.
 __device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, unsigned total, unsigned long long* bar,
                                                  unsigned parity, int cluster, int rank, bool lost) {
     if (cluster == 1) {
@@ -164,7 +176,10 @@ __device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, 
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         if (lane == 0) mbar_expect(bar, total - bytes);
-        if (lane < cluster && lane != rank && bytes) copy_to_peer(p, bytes, bar, lane);
+        if (lane < cluster && lane != rank) {
+            if (bytes) copy_to_peer(p, bytes, bar, lane);
+            else mbar_arrive_peer(bar, lane);
+        }
     }
     return lost || !mbar_wait(bar, parity);
 }
@@ -324,8 +339,8 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
     if (tid == 0) {
         xs[r.n] = V(0);
         ys[r.m] = V(0);
-        mbar_init(bar);
-        mbar_init(bar + 1);
+        mbar_init(bar, exchange_arrivals(r.idle_t, r.own_t));
+        mbar_init(bar + 1, exchange_arrivals(r.idle_a, r.own_a));
         mbar_init_visible();
     }
     const V tau = static_cast<V>(s.tau), sigma = static_cast<V>(s.sigma);
@@ -445,8 +460,8 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     for (int k = tid; k <= r.n; k += T) xs[k] = 0.0;
     for (int k = tid; k <= r.m; k += T) ys[k] = 0.0;
     if (tid == 0) {
-        mbar_init(bar);
-        mbar_init(bar + 1);
+        mbar_init(bar, exchange_arrivals(r.idle_t, r.own_t));
+        mbar_init(bar + 1, exchange_arrivals(r.idle_a, r.own_a));
         mbar_init_visible();
     }
     const int rank = static_cast<int>(blockIdx.x) % a.cluster;
@@ -748,7 +763,11 @@ inline void res_deal(const std::array<ResHist, 2>& H, int C, ResDeal& D) {
             pos += (own[c] + 3) & ~3;
             if (sd == 0) D.cta[c].pairs_t = D.cta[c].pairs;
         }
-        for (ResCta& k : D.cta) (sd == 0 ? k.n : k.m) = pos;
+        const int idle = static_cast<int>(std::count(own.begin(), own.end(), 0));
+        for (ResCta& k : D.cta) {
+            (sd == 0 ? k.n : k.m) = pos;
+            (sd == 0 ? k.idle_t : k.idle_a) = idle;
+        }
         for (auto& e : it) e.pos0 = (sd == 0 ? D.cta[e.cta].pos_t0 : D.cta[e.cta].pos_a0) + e.own0;
     }
 }
