@@ -14,10 +14,10 @@
 //     its share to every other one with a bulk copy between shared memories,
 //     which counts its bytes on the receiver's mbarrier; the receiver starts
 //     its next half when all shares are in.  A CTA that owns nothing on a side
-//     (few rows, many columns) arrives on the peers' mbarriers instead.  So a
-//     share of iteration k + 1 cannot overtake one of iteration k: it depends
-//     on the receiver's own share or arrival of the half in between, sent after
-//     its last read and after all of its shares of iteration k were in.
+//     (few rows, many columns) sends 16 bytes that nobody reads.  So a share of
+//     iteration k + 1 cannot overtake one of iteration k: it depends on the
+//     receiver's own share of the half in between, sent after its last read and
+//     after all of its shares of iteration k were in.
 //
 // Layout ("slices").  Rows are reduced by groups of G = 2^lg lanes, lane g of
 // a group adding entries g, g + G, ... of its row in order, then the groups'
@@ -78,7 +78,19 @@ struct ResClass {
     size_t smem = 0;
 };
 
-constexpr size_t kResBarBytes = 16;  // two mbarriers
+constexpr size_t kResBarBytes = 32;  // two mbarriers, and the 16 bytes of a CTA without a share
+constexpr unsigned kResIdleBytes = 16;
+
+// Bytes of a share of `own` entries in the exchange, and of all shares of a
+// vector of n positions of which `idle` CTAs own none.
+template <class V>
+__host__ __device__ inline unsigned share_bytes(int own) {
+    return own ? static_cast<unsigned>(sizeof(V)) * ((own + 3) & ~3) : kResIdleBytes;
+}
+template <class V>
+__host__ __device__ inline unsigned share_total(int n, int idle) {
+    return static_cast<unsigned>(sizeof(V)) * n + kResIdleBytes * idle;
+}
 
 template <class V>
 __host__ __device__ inline size_t res_vec_bytes(int n, int m, int own_t, int own_a) {
@@ -112,18 +124,10 @@ __device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
     return r;
 }
 
-// Arrivals that end a phase of a vector's mbarrier, next to the bytes announced
-// with the CTA's own: that one, and one of every other CTA that owns none of
-// the vector (`idle` of the cluster; `own`: this CTA's entries).
-__host__ __device__ inline int exchange_arrivals(int idle, int own) { return 1 + idle - (own == 0 ? 1 : 0); }
-__device__ __forceinline__ void mbar_init(unsigned long long* b, int arrivals) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b))),
-                 "r"(arrivals)
+// mbarriers of one arrival (the CTA's own) plus the bytes announced with it.
+__device__ __forceinline__ void mbar_init(unsigned long long* b) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b)))
                  : "memory");
-}
-// Arrival on the same mbarrier of CTA `rank`.
-__device__ __forceinline__ void mbar_arrive_peer(unsigned long long* b, int rank) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(b, rank)) : "memory");
 }
 __device__ __forceinline__ void mbar_init_visible() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect(unsigned long long* b, unsigned bytes) {
@@ -160,11 +164,10 @@ __device__ __forceinline__ void copy_to_peer(const void* p, unsigned bytes, unsi
 // Shared-memory writes of this thread, before a bulk copy reads them.
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// End of a half iteration: this CTA's share `p` of a gathered vector (or an
-// arrival, if it has none) goes to every other CTA of the cluster, and theirs
-// are awaited (`total`: the vector's bytes; `bar`: its mbarrier, at the phase
-// of `parity`).  Returns `lost`, or whether the wait ran out; once lost, later
-// waits are skipped.
+// End of a half iteration: this CTA's share `p` of a gathered vector goes to
+// every other CTA of the cluster, and theirs are awaited (`total`: all shares'
+// bytes; `bar`: its mbarrier, at the phase of `parity`).  Returns `lost`, or
+// whether the wait ran out; once lost, later waits are skipped.
 __device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, unsigned total, unsigned long long* bar,
                                                  unsigned parity, int cluster, int rank, bool lost) {
     if (cluster == 1) {
@@ -176,10 +179,7 @@ __device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, 
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         if (lane == 0) mbar_expect(bar, total - bytes);
-        if (lane < cluster && lane != rank) {
-            if (bytes) copy_to_peer(p, bytes, bar, lane);
-            else mbar_arrive_peer(bar, lane);
-        }
+        if (lane < cluster && lane != rank) copy_to_peer(p, bytes, bar, lane);
     }
     return lost || !mbar_wait(bar, parity);
 }
@@ -339,16 +339,20 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
     if (tid == 0) {
         xs[r.n] = V(0);
         ys[r.m] = V(0);
-        mbar_init(bar, exchange_arrivals(r.idle_t, r.own_t));
-        mbar_init(bar + 1, exchange_arrivals(r.idle_a, r.own_a));
+        mbar_init(bar);
+        mbar_init(bar + 1);
         mbar_init_visible();
     }
     const V tau = static_cast<V>(s.tau), sigma = static_cast<V>(s.sigma);
     cp_async_wait_all();
     const int rank = static_cast<int>(blockIdx.x) % a.cluster;
-    const unsigned bytes_x = sizeof(V) * r4(r.own_t), bytes_y = sizeof(V) * r4(r.own_a);
+    const unsigned bytes_x = share_bytes<V>(r.own_t), bytes_y = share_bytes<V>(r.own_a);
+    const unsigned total_x = share_total<V>(r.n, r.idle_t), total_y = share_total<V>(r.m, r.idle_a);
+    const void* const idle = smem + kResBarBytes - kResIdleBytes;
+    const void* const mine_x = r.own_t ? xs + r.pos_t0 : idle;
+    const void* const mine_y = r.own_a ? ys + r.pos_a0 : idle;
     bool lost = false;
-    auto exchange = [&](const V* p, unsigned bytes, unsigned total, int b, int it) {
+    auto exchange = [&](const void* p, unsigned bytes, unsigned total, int b, int it) {
         lost = cluster_exchange(p, bytes, total, bar + b, it & 1, a.cluster, rank, lost);
     };
     if (a.cluster > 1) cluster_sync();  // every CTA has started and holds its share
@@ -385,7 +389,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
                 xs[e.pos0 + grp] = V(2) * v - xk;
             }
         }
-        exchange(xs + r.pos_t0, bytes_x, sizeof(V) * r.n, 0, it);
+        exchange(mine_x, bytes_x, total_x, 0, it);
         for (int q = r.ns_t + warp; q < r.ns_t + r.ns_a; q += W) {  // dual half (DualEpi)
             const ResSlice e = sl[q];
             const int np = e.meta & 0xff, lg = (e.meta >> 8) & 0xf, nr = e.meta >> 12, grp = min(lane >> lg, nr - 1);
@@ -403,7 +407,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
                 ys[e.pos0 + grp] = v;
             }
         }
-        exchange(ys + r.pos_a0, bytes_y, sizeof(V) * r.m, 1, it);
+        exchange(mine_y, bytes_y, total_y, 1, it);
     }
     if (lost) {  // the solve stops at the coming check and reports the error
         atomicExch(a.error, 1);
@@ -460,12 +464,16 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     for (int k = tid; k <= r.n; k += T) xs[k] = 0.0;
     for (int k = tid; k <= r.m; k += T) ys[k] = 0.0;
     if (tid == 0) {
-        mbar_init(bar, exchange_arrivals(r.idle_t, r.own_t));
-        mbar_init(bar + 1, exchange_arrivals(r.idle_a, r.own_a));
+        mbar_init(bar);
+        mbar_init(bar + 1);
         mbar_init_visible();
     }
     const int rank = static_cast<int>(blockIdx.x) % a.cluster;
-    const unsigned bytes_x = 8 * r4(r.own_t), bytes_y = 8 * r4(r.own_a);
+    const unsigned bytes_x = share_bytes<double>(r.own_t), bytes_y = share_bytes<double>(r.own_a);
+    const unsigned total_x = share_total<double>(r.n, r.idle_t), total_y = share_total<double>(r.m, r.idle_a);
+    const void* const idle = smem + kResBarBytes - kResIdleBytes;
+    const void* const mine_x = r.own_t ? xs + r.pos_t0 : idle;
+    const void* const mine_y = r.own_a ? ys + r.pos_a0 : idle;
     cp_async_wait_all();
     if (a.cluster > 1) cluster_sync();
     else __syncthreads();
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     bool lost = false;
     double lambda = 0.0;
     for (int it = 0; it <= a.iters; ++it) {
-        lost = cluster_exchange(xs + r.pos_t0, bytes_x, 8u * r.n, bar, it & 1, a.cluster, rank, lost);
+        lost = cluster_exchange(mine_x, bytes_x, total_x, bar, it & 1, a.cluster, rank, lost);
         double s = 0.0;
         for (int k = tid; k < r.n; k += T) s += xs[k] * xs[k];
         s = warp_sum(s);
@@ -492,7 +500,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
             const double t = slice_sum<double, double>(e.pair0, e.meta & 0xff, lg, idx, val, xs, lane);
             if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < (e.meta >> 12)) ys[e.pos0 + (lane >> lg)] = t / nz;
         }
-        lost = cluster_exchange(ys + r.pos_a0, bytes_y, 8u * r.m, bar + 1, it & 1, a.cluster, rank, lost);
+        lost = cluster_exchange(mine_y, bytes_y, total_y, bar + 1, it & 1, a.cluster, rank, lost);
         for (int q = warp; q < r.ns_t; q += W) {
             const ResSlice e = sl[q];
             const int lg = (e.meta >> 8) & 0xf;

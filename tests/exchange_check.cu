@@ -4,7 +4,7 @@
 // halves of several iterations on the shares that res_deal gives, with every
 // message delayed at random: no message of one iteration may reach a barrier
 // whose phase belongs to another, and every CTA gets to the end.  The same
-// model without the arrivals of CTAs that own nothing finds the overtaking that
+// model without the shares of CTAs that own nothing finds the overtaking that
 // they prevent.
 #include <cstdio>
 #include <random>
@@ -16,34 +16,30 @@
 using namespace gb;
 
 struct Bar {
-    int count, pending;
+    int pending = 1;   // the CTA's own arrival
     long long tx = 0;  // bytes announced and not yet in
     int phase = 0;
     void settle() {
         if (pending == 0 && tx == 0) {
-            pending = count;
+            pending = 1;
             ++phase;
         }
     }
 };
 struct Message {
     int to, half;
-    long long bytes;  // 0: an arrival
+    long long bytes;
 };
 
 // Whether a run of `iters` iterations went wrong: 1 overtaking, 2 no end.
-static int run(const std::vector<ResCta>& cta, int iters, bool arrivals, std::mt19937& rng) {
+static int run(const std::vector<ResCta>& cta, int iters, bool shares, std::mt19937& rng) {
     const int C = static_cast<int>(cta.size());
     auto own = [&](int c, int side) { return side == 0 ? cta[c].own_t : cta[c].own_a; };
-    auto bytes = [&](int c, int side) { return 4LL * ((own(c, side) + 3) & ~3); };
-    const long long total[2] = {4LL * cta[0].n, 4LL * cta[0].m};
+    // `shares`: CTAs that own nothing take part too
+    auto bytes = [&](int c, int side) { return shares || own(c, side) ? static_cast<long long>(share_bytes<float>(own(c, side))) : 0; };
+    const long long total[2] = {share_total<float>(cta[0].n, shares ? cta[0].idle_t : 0),
+                                share_total<float>(cta[0].m, shares ? cta[0].idle_a : 0)};
     std::vector<std::array<Bar, 2>> bar(C);
-    for (int c = 0; c < C; ++c)
-        for (int side = 0; side < 2; ++side) {
-            const int idle = side == 0 ? cta[c].idle_t : cta[c].idle_a;
-            Bar& b = bar[c][side];
-            b.count = b.pending = arrivals ? exchange_arrivals(idle, own(c, side)) : 1;
-        }
     std::vector<int> half(C, 0), sent(C, 0);  // half c is in; whether it has sent
     std::vector<Message> air;
     auto done = [&] {
@@ -61,8 +57,7 @@ static int run(const std::vector<ResCta>& cta, int iters, bool arrivals, std::mt
             if (msg.to == slow && rng() % 64 != 0) continue;
             Bar& b = bar[msg.to][msg.half & 1];
             if (b.phase != msg.half >> 1) return 1;
-            if (msg.bytes) b.tx -= msg.bytes;
-            else --b.pending;
+            b.tx -= msg.bytes;
             b.settle();
             air[k] = air.back();
             air.pop_back();
@@ -77,7 +72,7 @@ static int run(const std::vector<ResCta>& cta, int iters, bool arrivals, std::mt
             b.tx += total[side] - bytes(c, side);
             --b.pending;
             for (int p = 0; p < C; ++p)
-                if (p != c && (bytes(c, side) || arrivals)) air.push_back({p, half[c], bytes(c, side)});
+                if (p != c && bytes(c, side)) air.push_back({p, half[c], bytes(c, side)});
             b.settle();
         }
         if (b.phase > half[c] >> 1) {
@@ -134,10 +129,10 @@ int main() {
             without += run(D.cta, 5, false, rng) != 0;
         }
         if (wrong || (without > 0) != (idle[0] + idle[1] > 0)) {
-            std::printf("FAIL %s: %d of 300 runs overtaken, %d without arrivals\n", c.name, wrong, without);
+            std::printf("FAIL %s: %d of 300 runs overtaken, %d without the idle CTAs' shares\n", c.name, wrong, without);
             bad = 1;
         } else {
-            std::printf("ok %s: C=%d, %d + %d own nothing, overtaken without arrivals in %d of 300 runs\n", c.name, c.C,
+            std::printf("ok %s: C=%d, %d + %d own nothing, overtaken without their shares in %d of 300 runs\n", c.name, c.C,
                         idle[0], idle[1], without);
         }
     }
