@@ -176,6 +176,7 @@ void qx_dplr_f64(Problem& P, const double* x, double* out, cudaStream_t s);
 constexpr int kPowerIters = 50;
 void prepare_power(Problem& P);
 void launch_power_chip(Problem& P, cudaStream_t s);
+void order_resident(Problem& P);
 bool all_resident(const Problem& P) {
     const ResPlan& R = P.res[1];
     return R.any() && R.list_na[1] == 0;
@@ -508,10 +509,11 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
                                                                                   P->F64.get(), P->D64.get());
     }
     if (P->has_q) power_iteration(*P, true, s);
-    // ||A'|| (scaling.cpp:131-155): on chip for the resident instances, whatever
-    // shares their batch
+    // ||A'|| (scaling.cpp:131-155): on chip for the resident instances, the same
+    // bits whatever shares their batch
     prepare_power(*P);
     power_iteration(*P, false, s);
+    order_resident(*P);
     tr.mark("power iteration");
     // w0 from the scaled data (pdhg_impl.hpp:258-261)
     inst_reduce(*P, false, Sq{P->c.get()}, S_CN, PostSqrt{}, s);
@@ -808,10 +810,23 @@ template <class M, class V>
 void ensure_resident_values(Problem& P) {
     ResPlan& R = P.res[sizeof(V) == 8];
     if (!R.any()) return;
-    auto pack = [&](auto& buf, auto src) { pack_values(P, buf, R.pairs, R.slot_t, R.slot_a, R.at, R.step_t, R.step_a, src); };
+    auto pack = [&](auto& buf, auto src) { pack_values(P, buf, R.pairs, R.slot_t, R.slot_a, R.at, R.ordered ? R.step_t : nullptr,
+                                                     R.ordered ? R.step_a : nullptr, src); };
     if constexpr (std::is_same<M, double>::value) pack(R.val64, [](const DevMat& A) { return A.val64.get(); });
     else if constexpr (std::is_same<M, float>::value) pack(R.val32, [](const DevMat& A) { return A.val32.get(); });
     else pack(R.valbf, [](const DevMat& A) { return A.valbf.get(); });
+}
+
+// The FP64 plan's entries in k_res_order's order.
+void order_resident(Problem& P) {
+    ResPlan& R = P.res[1];
+    if (!R.any() || R.ordered) return;
+    const ResOrderArgs a{{{R.col_at, P.AT.ptr.get(), P.AT.idx.get(), P.AT.val64.get(), R.pos_a, R.step_t},
+                          {R.row_at, P.A.ptr.get(), P.A.idx.get(), P.A.val64.get(), R.pos_t, R.step_a}},
+                         reinterpret_cast<unsigned short*>(R.idx), R.val64.get()};
+    k_res_order<<<div_up(R.nslices, 4), 128, 0, P.stream>>>(R.nslices, R.at, a);
+    GB_CUDA(cudaGetLastError());
+    R.ordered = true;
 }
 
 // Which instances run on chip with vectors of type V (index w), in clusters
@@ -821,9 +836,11 @@ void ensure_resident_values(Problem& P) {
 // SMs by work (a lone LP spreads over 16, an instance of a large batch takes
 // the fewest CTAs that hold it), but no CTA gets fewer than kResMinSlices
 // slices, where the barrier outweighs the work.
+// `order` = false leaves the entries of an FP64 plan in the matrix's order, for
+// the power iteration, until order_resident.
 constexpr int kResMinSlices = 4;
 template <class V>
-void ensure_resident(Problem& P) {
+void ensure_resident(Problem& P, bool order = true) {
     constexpr int w = sizeof(V) == 8;
     constexpr size_t sm = sizeof(V);  // FP64 vectors: sized for the FP64 matrix
     ResPlan& R = P.res[w];
@@ -979,6 +996,7 @@ void ensure_resident(Problem& P) {
         T.add(p.k, hist[p.at], p.deal, P.col_off[p.k], P.col_off[p.k + 1], P.row_off[p.k], P.row_off[p.k + 1]);
     }
     R.pairs = T.pairs;
+    R.nslices = static_cast<int>(T.at.size());
     cudaStream_t s = P.stream;
     // by matrix type: FP64 vectors meet either (the FP32 matrix in Dynamic solves)
     std::vector<RowBlock> la[2], lt[2];
@@ -1020,16 +1038,14 @@ void ensure_resident(Problem& P) {
     k_res_rank<<<ns, 32, 0, s>>>(R.sides_a, P.A.ptr.get(), R.lg_a, R.at, R.slot_a, R.pos_a, R.row_at);
     k_res_fill<<<static_cast<int>(T.cta.size()), kThreads, 0, s>>>(R.cta, R.idx);
     unsigned short* idx16 = reinterpret_cast<unsigned short*>(R.idx);
-    if (w) {
-        ResOrderArgs o{{{R.col_at, P.AT.ptr.get(), P.AT.idx.get(), R.pos_a, R.step_t},
-                        {R.row_at, P.A.ptr.get(), P.A.idx.get(), R.pos_t, R.step_a}}};
-        const int ns = static_cast<int>(T.at.size());
-        k_res_order<<<div_up(ns, 4), 128, 0, s>>>(ns, R.at, o);
+    if (w && order) {
+        order_resident(P);
+    } else {
+        k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t, R.at,
+                                                                 R.pos_a, idx16);
+        k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a, R.at,
+                                                                 R.pos_t, idx16);
     }
-    k_res_entries<<<elem_grid(P.n, P.sms), kThreads, 0, s>>>(P.n, P.AT.ptr.get(), P.AT.idx.get(), R.slot_t, R.at,
-                                                             R.pos_a, R.step_t, idx16);
-    k_res_entries<<<elem_grid(P.m, P.sms), kThreads, 0, s>>>(P.m, P.A.ptr.get(), P.A.idx.get(), R.slot_a, R.at,
-                                                             R.pos_t, R.step_a, idx16);
     GB_CUDA(cudaGetLastError());
     if (trace_enabled())
         for (const ResClass& c : R.classes)
@@ -1111,14 +1127,14 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
 
 // The FP64 plan, ahead of the power iteration that runs on it.
 void prepare_power(Problem& P) {
-    ensure_resident<double>(P);
+    ensure_resident<double>(P, false);
     ensure_resident_values<double, double>(P);
 }
 void launch_power_chip(Problem& P, cudaStream_t s) {
     const ResPlan& R = P.res[1];
     for (const ResClass& c : R.classes) {
-        const PowerArgs a{R.cta + c.cta0, R.slices, R.idx, R.val64.get(), P.scal.get(), kScal, S_PW_LAMBDA,
-                          P.phase_flags.get() + P.count, kPowerIters, c.cluster};
+        const PowerArgs a{R.cta + c.cta0, R.slices, R.idx, R.val64.get(), R.pos_t, P.d_col_off.get(),
+                          P.scal.get(), kScal, S_PW_LAMBDA, P.phase_flags.get() + P.count, kPowerIters, c.cluster};
         cudaLaunchAttribute attr[1];
         const cudaLaunchConfig_t cfg = resident_config(c, attr, s);
         GB_CUDA(cudaLaunchKernelEx(&cfg, c.threads == 256 ? k_power_chip<256> : c.threads == 512 ? k_power_chip<512> : k_power_chip<1024>, a));

@@ -24,8 +24,10 @@
 // shuffle tree -- for FP32 vectors exactly spmv_run's order with the row
 // block's own lg, so an FP32 iterate has the same bits on either path.  (FP64
 // kernels stream with the segmented order of spmv_run_seg; here lg comes from
-// the row's length alone, so an instance's result does not depend on what
-// shares its batch.)  A slice is 32 >> lg rows, one warp; rows are sorted by
+// the row's length, and a lane takes its entries as their positions' banks
+// allow, which follow the cluster's size: FP64 iterates of an instance may
+// differ in their last bits between batches.  Its norm and FP32 iterates do
+// not.)  A slice is 32 >> lg rows, one warp; rows are sorted by
 // their number of lane steps, so slices carry almost no padding, and a
 // slice's entries are stored step-major in pairs: for pair t, 32 words of two
 // 16-bit column positions and 32 pairs of values -- conflict-free reads
@@ -429,7 +431,9 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
 // Power iteration on A'^T A' (scaling.cpp:131-155) of the resident instances on
 // the FP64 plan: 50 steps in one launch instead of 200 launches (0.6 - 1 ms of
 // a small LP's set-up; 0.1 - 0.2 ms here).  z is in xs and w in ys; after z's
-// exchange every CTA forms ||z|| over all of it in the same order.
+// exchange every CTA forms ||z|| over all of it, in the order of the columns
+// (k_seg_red's), not of their positions: the norm, and with it the step sizes,
+// must not depend on the cluster's size, which follows what shares the batch.
 inline size_t power_smem_bytes(const ResCta& c) {
     return res_smem_bytes<double, double>(c.ns_t + c.ns_a, c.pairs, c.n, c.m, 0, 0) + 8 * 32;
 }
@@ -438,6 +442,8 @@ struct PowerArgs {
     const ResSlice* slices;
     const unsigned* idx;
     const double* val;
+    const unsigned short* pos_t;  // column -> position
+    const int* col_off;           // instance -> first column
     double* scal;          // per instance rows of kScal; [lambda] is written
     int scal_stride, lambda;
     int* error;
@@ -460,10 +466,9 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     for (int k = tid; k < r.ns_t + r.ns_a; k += T) cp_async16(sl + k, a.slices + r.slice0 + k);
     for (int k = tid; k < 8 * r.pairs; k += T) cp_async16(idx + 4 * k, a.idx + 32 * r.pair0 + 4 * k);
     for (int k = tid; k < 32 * r.pairs; k += T) cp_async16(val + 2 * k, a.val + 64 * r.pair0 + 2 * k);
-    // places between two shares and the zero slots stay 0: they add nothing to ||z||
-    for (int k = tid; k <= r.n; k += T) xs[k] = 0.0;
-    for (int k = tid; k <= r.m; k += T) ys[k] = 0.0;
     if (tid == 0) {
+        xs[r.n] = 0.0;
+        ys[r.m] = 0.0;
         mbar_init(bar);
         mbar_init(bar + 1);
         mbar_init_visible();
@@ -474,6 +479,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     const void* const idle = smem + kResBarBytes - kResIdleBytes;
     const void* const mine_x = r.own_t ? xs + r.pos_t0 : idle;
     const void* const mine_y = r.own_a ? ys + r.pos_a0 : idle;
+    const int c0 = a.col_off[r.inst], c1 = a.col_off[r.inst + 1];
     cp_async_wait_all();
     if (a.cluster > 1) cluster_sync();
     else __syncthreads();
@@ -483,13 +489,19 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     for (int it = 0; it <= a.iters; ++it) {
         lost = cluster_exchange(mine_x, bytes_x, total_x, bar, it & 1, a.cluster, rank, lost);
         double s = 0.0;
-        for (int k = tid; k < r.n; k += T) s += xs[k] * xs[k];
-        s = warp_sum(s);
-        if (lane == 0) red[warp] = s;
+        if (warp < kWarps) {
+#pragma unroll 4
+            for (int j = c0 + tid; j < c1; j += kThreads) {
+                const double z = xs[a.pos_t[j]];
+                s += z * z;
+            }
+            s = warp_sum(s);
+            if (lane == 0) red[warp] = s;
+        }
         __syncthreads();
         double nz = 0.0;
 #pragma unroll
-        for (int w = 0; w < W; ++w) nz += red[w];
+        for (int w = 0; w < kWarps; ++w) nz += red[w];
         nz = sqrt(nz);
         if (it > 0 && nz != 0.0) lambda = nz;
         if (it == a.iters || nz == 0.0) break;  // the same in every CTA
@@ -536,6 +548,7 @@ struct ResSliceAt {                        // slice list entry: where the slice 
     long long pair0;                       // global first pair
     int meta, pos0;
     int at0, side;                         // its instance's first entry of the side's position -> row list; 0: A^T
+    int zero;                              // the gathered vector's zero slot
 };
 
 // One warp per side walks its rows in order and gives every row its slot
@@ -587,16 +600,22 @@ static __global__ void k_res_fill(const ResCta* __restrict__ cta, unsigned* __re
 // gather from as many different pairs of banks as can be had (the order of a
 // lane's sum is free there; random positions take 3.1 wavefronts a half, these
 // ~2).  One warp per slice: lane by lane, both halves side by side, each entry
-// goes to the free step whose bank pair is least used so far.  Measured, FP64:
+// goes to the free step whose bank pair is least used so far, with its position
+// and (`val` given) its value.  Positions, and so the order of the sums, follow
+// the cluster's size, which follows what shares the batch; the power iteration
+// therefore runs before, on entries in the matrix's order.  Measured, FP64:
 // LP 2000 x 5000 2.25 -> 2.18 ms, 37 LPs 2.86 -> 2.76, 64 branching children
 // 161 -> 155.
 struct ResOrderSide {
     const int *at, *ptr, *col;          // position -> row, the rows
+    const double* val;
     const unsigned short* pos_other;    // positions of the gathered vector
     unsigned char* step;
 };
 struct ResOrderArgs {
     ResOrderSide side[2];
+    unsigned short* idx;
+    double* val;                        // packed values, or nullptr: positions alone
 };
 static __global__ void __launch_bounds__(128) k_res_order(int nslices, const ResSliceAt* __restrict__ slices,
                                                           const __grid_constant__ ResOrderArgs a) {
@@ -615,11 +634,16 @@ static __global__ void __launch_bounds__(128) k_res_order(int nslices, const Res
         p0 = d.ptr[r];
         len = d.ptr[r + 1] - p0;
     }
+    auto put = [&](int t, int pos, double v) {
+        const long long z = (e.pair0 + (t >> 1)) * 64 + 2 * lane + (t & 1);
+        a.idx[z] = static_cast<unsigned short>(pos);
+        if (a.val) a.val[z] = v;
+    };
+    unsigned taken = 0u;
     for (int l = 0; l < 16; ++l) {
         if ((lane & 15) == l) {
-            unsigned taken = 0u;
             for (int k = lane & (G - 1); k < len; k += G) {
-                const int bank = d.pos_other[d.col[p0 + k]] & 15;
+                const int pos = d.pos_other[d.col[p0 + k]], bank = pos & 15;
                 int best = 0, least = 255;
                 for (int t = 0; t < steps; ++t) {
                     const int u = load[w][half][t][bank];
@@ -631,10 +655,13 @@ static __global__ void __launch_bounds__(128) k_res_order(int nslices, const Res
                 taken |= 1u << best;
                 ++load[w][half][best][bank];
                 d.step[p0 + k] = static_cast<unsigned char>(best);
+                put(best, pos, a.val ? d.val[p0 + k] : 0.0);
             }
         }
         __syncwarp();
     }
+    for (int t = 0; t < steps; ++t)
+        if (!(taken >> t & 1u)) put(t, e.zero, 0.0);
 }
 
 // Entries of the rows of one side: positions (from the other side's
@@ -642,14 +669,14 @@ static __global__ void __launch_bounds__(128) k_res_order(int nslices, const Res
 static __global__ void k_res_entries(int rows, const int* __restrict__ ptr, const int* __restrict__ col,
                                      const int* __restrict__ slot, const ResSliceAt* __restrict__ slices,
                                      const unsigned short* __restrict__ pos_other,
-                                     const unsigned char* __restrict__ step, unsigned short* __restrict__ idx) {
+                                     unsigned short* __restrict__ idx) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
         const int sr = slot[r];
         if (sr < 0) continue;  // the row's instance is not resident
         const ResSliceAt e = slices[sr >> 5];
         const int lg = (e.meta >> 8) & 0xf, G = 1 << lg, p0 = ptr[r], len = ptr[r + 1] - p0;
         for (int k = 0; k < len; ++k) {
-            const int t = step ? step[p0 + k] : k >> lg, lane = ((sr & 31) << lg) + (k & (G - 1));
+            const int t = k >> lg, lane = ((sr & 31) << lg) + (k & (G - 1));
             idx[(e.pair0 + (t >> 1)) * 64 + 2 * lane + (t & 1)] = pos_other[col[p0 + k]];
         }
     }
@@ -817,7 +844,7 @@ struct ResTables {
                 if (s.slice0[e.lg] < 0) s.slice0[e.lg] = static_cast<int>(at.size());
                 const ResCta& k = cta[c0 + e.cta];
                 const int meta = e.pairs | e.lg << 8 | e.rows << 12;
-                at.push_back({k.pair0 + e.pair0, meta, e.pos0, positions[sd], sd});
+                at.push_back({k.pair0 + e.pair0, meta, e.pos0, positions[sd], sd, sd == 0 ? k.m : k.n});
                 slices[k.slice0 + (sd == 0 ? 0 : k.ns_t) + e.ord] = {e.pair0, meta, e.own0, e.pos0};
             }
             sides[sd].push_back(s);
@@ -890,10 +917,12 @@ struct ResPlan {
     unsigned short *pos_t = nullptr, *pos_a = nullptr;
     unsigned char *lg_t = nullptr, *lg_a = nullptr;      // FP32
     unsigned char *step_t = nullptr, *step_a = nullptr;  // FP64: k_res_order
+    bool ordered = false;                                // whether the entries lie in that order
     DevBuf<float> val32;
     DevBuf<double> val64;
     DevBuf<__nv_bfloat16> valbf;
     long long pairs = 0;
+    int nslices = 0;
     // Row blocks of the other instances, which the streaming kernels run
     // (nothing: every instance is resident), by matrix type (0: FP32 / BF16,
     // 1: FP64): a block's bitmap, slots and counter are those of the schedule
