@@ -307,6 +307,14 @@ int load_mode_override() {
 
 void prebuild_graphs(Problem& P, const gb_options* opt);
 
+// After a synchronisation of the problem's stream.
+void release_plan_scratch(Problem& P) {
+    if (trace_enabled() && (!P.plan_scratch.pinned.empty() || !P.plan_scratch.dev.empty()))
+        std::fprintf(stderr, "[gb trace] plan scratch given back: %zu pinned blocks, %zu B of device memory\n",
+                     P.plan_scratch.pinned.size(), P.plan_scratch.dev_bytes());
+    P.plan_scratch.release();
+}
+
 // Upload + device setup (scale_lp + estimate_norm + run_pdhg's start point)
 // of `count` instances.
 Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
@@ -553,6 +561,7 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     GB_CUDA(cudaStreamSynchronize(s));
     GB_CUDA(cudaGetLastError());
     if (P->phase_flags_host[count]) throw Error(GB_ERR_CUDA, "an exchange between the CTAs of a cluster timed out");
+    release_plan_scratch(*P);
     P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return P.release();
 }
@@ -1028,7 +1037,7 @@ void ensure_resident(Problem& P, bool order = true) {
         arena.raw(R.step_t, P.A.nnz);
         arena.raw(R.step_a, P.A.nnz);
     }
-    arena.commit(R.mem, P.pinned, s);
+    arena.commit(R.mem, P.plan_scratch, s);
     if (w == 0) {
         k_res_row_lg<<<st.nb, kThreads, 0, s>>>(st.nb, st.blocks.get(), R.lg_t);
         k_res_row_lg<<<sa.nb, kThreads, 0, s>>>(sa.nb, sa.blocks.get(), R.lg_a);
@@ -1232,7 +1241,7 @@ void build_grid(Problem& P, GridPlan& R) {
             sides[sd].push_back(S);
         }
     }
-    PlanArena first;
+    PlanArena first, packing;
     first.host(R.at, at);
     for (int sd = 0; sd < 2; ++sd) {
         const size_t rows = mats[sd]->rows, map = static_cast<size_t>(kGridCtas) * div_up(mats[sd]->cols, 32);
@@ -1241,11 +1250,13 @@ void build_grid(Problem& P, GridPlan& R) {
         first.raw(R.slot[sd], rows);
         first.raw(R.pos[sd], rows);
         if (w == 0) first.raw(R.lg[sd], rows);
-        first.raw(R.bits[sd], map);
-        first.raw(R.before[sd], map);
+        packing.raw(R.bits[sd], map);
+        packing.raw(R.before[sd], map);
         first.raw(R.count[sd], kGridCtas);
     }
-    first.commit(R.mem[0], P.pinned, s);
+    P.plan_scratch.dev.emplace_back();
+    packing.commit(P.plan_scratch.dev.back(), P.plan_scratch, s);
+    first.commit(R.mem[0], P.plan_scratch, s);
     std::vector<int> count[2], list0[2];
     for (int sd = 0; sd < 2; ++sd) {
         const int rows = mats[sd]->rows, words = div_up(mats[sd]->cols, 32);
@@ -1327,7 +1338,7 @@ void build_grid(Problem& P, GridPlan& R) {
     second.raw(R.gx, words * P.n);
     second.raw(R.gy, words * P.m);
     second.raw(R.sync, 3);
-    second.commit(R.mem[1], P.pinned, s);
+    second.commit(R.mem[1], P.plan_scratch, s);
     GB_CUDA(cudaMemsetAsync(R.sync, 0, 3 * sizeof(unsigned), s));
     GB_CUDA(cudaMemsetAsync(R.gx, 0, 8 * words * P.n, s));  // tags start at 1
     GB_CUDA(cudaMemsetAsync(R.gy, 0, 8 * words * P.m, s));
@@ -1791,6 +1802,7 @@ void run_phase(Problem& P, const gb_options* opt, double tol, int stall_exit, in
     }
     P.launches += 1 + bodies * per_body;
     GB_CUDA(cudaGetLastError());
+    release_plan_scratch(P);
     if (P.phase_flags_host[P.count]) throw Error(GB_ERR_CUDA, "an exchange between the CTAs of a cluster timed out");
 }
 
@@ -2066,6 +2078,7 @@ void by_level(int level, Problem& P, F&& f) {
 void rebuild_schedules(Problem& P, int w) {
     cudaStream_t s = P.stream;
     GB_CUDA(cudaStreamSynchronize(s));
+    release_plan_scratch(P);
     for (auto& g : P.graphs) g.reset();
     for (ResPlan& r : P.res) r = ResPlan{};  // packed by these schedules' lanes per row
     for (GridPlan& r : P.grid) r = GridPlan{};

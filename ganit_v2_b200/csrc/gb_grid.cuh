@@ -325,7 +325,7 @@ struct GridPlan {
     ResSliceAt* at = nullptr;
     ResSide* sides[2] = {};                        // A^T, A
     int *list[2] = {}, *src[2] = {}, *slot[2] = {}, *pos[2] = {};
-    unsigned* bits[2] = {};                        // packing scratch
+    unsigned* bits[2] = {};                        // packing alone: in Problem::plan_scratch, as `before`
     int *before[2] = {}, *count[2] = {}, *list0[2] = {};
     unsigned char* lg[2] = {};
     long long* pair0[2] = {};

@@ -134,7 +134,7 @@ struct Problem {
     VecSet<float> v32;
     VecSet<double> v64;
     DevBuf<SolveState> st;                // per instance
-    std::vector<void*> pinned;            // sources of the plans' copies
+    PlanScratch plan_scratch;             // of the plans made since the stream was last idle
     SolveState* st_host = nullptr;        // pinned mirror (count entries)
     DevBuf<int> phase_flags;              // per-instance flags uploaded for a phase; last entry: k_resident's error
     int* phase_flags_host = nullptr;      // pinned (count + 1)
@@ -172,7 +172,7 @@ struct Problem {
         free_batch.open = true;
         for (auto& g : graphs) g.reset();
         host_free(st_host);
-        for (void* p : pinned) host_free(p);
+        for (void* p : plan_scratch.pinned) host_free(p);
         host_free(phase_flags_host);
         if (stream) cudaStreamDestroy(stream);
     }

@@ -854,11 +854,30 @@ struct ResTables {
     }
 };
 
+// Pinned and device memory that a plan needs only while it is packed.
+struct PlanScratch {
+    std::vector<void*> pinned;  // sources of the plans' copies
+    std::vector<DevBuf<unsigned char>> dev;
+    size_t dev_bytes() const {
+        size_t b = 0;
+        for (const auto& d : dev) b += d.size();
+        return b;
+    }
+    // Gives it back; the stream that packed has to be idle.
+    void release() {
+        if (pinned.empty() && dev.empty()) return;
+        begin_free_batch();
+        for (void* p : pinned) host_free(p);
+        pinned.clear();
+        dev.clear();
+        end_free_batch();
+    }
+};
+
 // Device arrays of a plan in one allocation (a cudaMalloc each took longer
 // than packing a small LP), those filled by the host in one copy, those that
 // start as -1 in one memset.  The copy's source is pinned, so the host goes on
-// while earlier work of the stream runs; the caller frees it (host_free) with
-// the problem.
+// while earlier work of the stream runs; it stays in `scratch` until released.
 class PlanArena {
    public:
     template <class T>
@@ -869,7 +888,7 @@ class PlanArena {
     void ones(T*& p, size_t n) { add(reinterpret_cast<void**>(&p), n * sizeof(T), 1, nullptr); }
     template <class T>
     void raw(T*& p, size_t n) { add(reinterpret_cast<void**>(&p), n * sizeof(T), 2, nullptr); }
-    void commit(DevBuf<unsigned char>& mem, std::vector<void*>& pinned, cudaStream_t s) {
+    void commit(DevBuf<unsigned char>& mem, PlanScratch& scratch, cudaStream_t s) {
         size_t end[3], off = 0;
         for (int kind = 0; kind < 3; ++kind) {
             for (Item& i : items_)
@@ -880,8 +899,11 @@ class PlanArena {
             end[kind] = off;
         }
         mem.reset(std::max<size_t>(off, 256));
-        unsigned char* stage = static_cast<unsigned char*>(host_alloc(std::max<size_t>(end[0], 1)));
-        pinned.push_back(stage);
+        unsigned char* stage = nullptr;
+        if (end[0]) {
+            stage = static_cast<unsigned char*>(host_alloc(end[0]));
+            scratch.pinned.push_back(stage);
+        }
         for (const Item& i : items_) {
             *i.slot = mem.get() + i.off;
             if (i.kind == 0 && i.bytes) std::memcpy(stage + i.off, i.src, i.bytes);
