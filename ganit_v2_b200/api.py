@@ -554,7 +554,8 @@ class Problem:
         return mp.value, md.value, nl.value
 
     def autotune(self, iters: int = 50) -> dict:
-        """Pick the row-block cut by timing (gb_problem_autotune); solve once first."""
+        """Pick the row-block cut by timing (gb_problem_autotune); solve once first.
+        A level whose solves iterate on chip keeps the default cut."""
         bn, mr = np.zeros(2, dtype=np.int32), np.zeros(2, dtype=np.int32)
         t0, t1 = np.zeros(2), np.zeros(2)
         _check(self._lib.gb_problem_autotune(self._h, int(iters), _p(bn), _p(mr), _p(t0), _p(t1)))
@@ -662,7 +663,8 @@ class BatchSolver:
         return {"threads": t.value, "blocks_per_sm": b.value, "groups_A": g[0::2].copy(), "groups_AT": g[1::2].copy()}
 
     def autotune(self, iters: int = 30) -> dict:
-        """Pick row-split schedules per instance-size class by timing (gb_batch_autotune)."""
+        """Pick row-split schedules per instance-size class by timing (gb_batch_autotune).
+        A level whose solves run wholly on chip keeps the default cut."""
         k = len(self.lps)
         bn = np.zeros(2 * k, dtype=np.int32)
         mr = np.zeros(2 * k, dtype=np.int32)

@@ -1502,15 +1502,10 @@ struct Branches {
     }
 };
 
-// Body of the phase loop: check_every iterations, KKT check, restart.
-// use_cond = 0 when the body is launched from the host loop instead of the graph.
+// `ce` iterations of a body, on chip and streamed (iterate in buffer 0); `nl`
+// counts the launches.  Returns the number of branches that ran side by side.
 template <class M, class V>
-long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cudaStream_t s, int use_cond = 1) {
-    VecSet<V>& vs = Level<M, V>::vs(P);
-    long long nl = 0;
-    const bool odd = (ce & 1) != 0;
-    const V* xc = odd ? vs.x1.get() : vs.x0.get();
-    const V* yc = odd ? vs.y1.get() : vs.y0.get();
+int launch_iterations(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s, long long& nl) {
     const StreamBlocks sb = stream_blocks<M, V>(P);
     Branches br(s);
     for (const ResClass& c : P.res[sizeof(V) == 8].classes) {
@@ -1534,6 +1529,19 @@ long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cuda
         for (int k = 0; k < ce; ++k) launch_iteration<M, V>(P, vs, k, s, nl, nullptr, sb);
     }
     br.join();
+    return br.count;
+}
+
+// Body of the phase loop: check_every iterations, KKT check, restart.
+// use_cond = 0 when the body is launched from the host loop instead of the graph.
+template <class M, class V>
+long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cudaStream_t s, int use_cond = 1) {
+    VecSet<V>& vs = Level<M, V>::vs(P);
+    long long nl = 0;
+    const bool odd = (ce & 1) != 0;
+    const V* xc = odd ? vs.x1.get() : vs.x0.get();
+    const V* yc = odd ? vs.y1.get() : vs.y0.get();
+    const int branches = launch_iterations<M, V>(P, vs, ce, s, nl);
     if (P.has_q) launch_qx2<M, V>(P, vs, xc, s, nl);
     EvalArgs<M, V> ea = eval_args<M, V>(P, vs, xc, yc, kEvalCheck, P.has_q);
     ea.cond = cond;
@@ -1541,7 +1549,7 @@ long long capture_body(Problem& P, int ce, cudaGraphConditionalHandle cond, cuda
     const int grid = ea.A.nb + ea.AT.nb;
     auto eval = P.detect_unbounded && !P.has_q ? k_eval<M, V, 3, 3>  // third right-hand side of the A pass: the primal ray
                                                : k_eval<M, V, 2, 3>;
-    if (br.count > 1) eval<<<grid, kThreads, spmv_smem_bytes<3, V>(), s>>>(ea);  // joins several branches
+    if (branches > 1) eval<<<grid, kThreads, spmv_smem_bytes<3, V>(), s>>>(ea);  // joins several branches
     else launch_pdl(eval, grid, kThreads, spmv_smem_bytes<3, V>(), s, ea);
     nl += launch_decide<M, V>(P, ea, s, true);
     RestartArgs<V> ra{xc, yc, vs.x0.get(), vs.y0.get(), vs.xr.get(), vs.yr.get(), vs.sumx.get(), vs.sumy.get(),
@@ -1963,14 +1971,20 @@ struct Tag {
     using V = V_;
 };
 
+// Every instance active, iterating from the carried point.
+template <class M, class V>
+void enter_timing(Problem& P, VecSet<V>& vs) {
+    k_activate_all<<<div_up(P.count, kThreads), kThreads, 0, P.stream>>>(P.count, P.st.get());
+    k_phase_in<V><<<elem_grid(std::max(P.n, P.m), P.sms), kThreads, 0, P.stream>>>(
+        P.n, P.m, P.icol(), P.irow(), P.st.get(), P.x64.get(), P.y64.get(), P.x64.get(), P.y64.get(), 0,
+        vs.x0.get(), vs.y0.get(), vs.xr.get(), vs.yr.get(), vs.sumx.get(), vs.sumy.get());
+}
+
 template <class M, class V>
 void time_level(Problem& P, int iters, double* msp, double* msd, int64_t* launches) {
     cudaStream_t s = P.stream;
     VecSet<V>& vs = Level<M, V>::vs(P);
-    k_activate_all<<<div_up(P.count, kThreads), kThreads, 0, s>>>(P.count, P.st.get());
-    k_phase_in<V><<<elem_grid(std::max(P.n, P.m), P.sms), kThreads, 0, s>>>(
-        P.n, P.m, P.icol(), P.irow(), P.st.get(), P.x64.get(), P.y64.get(), P.x64.get(), P.y64.get(), 0,
-        vs.x0.get(), vs.y0.get(), vs.xr.get(), vs.yr.get(), vs.sumx.get(), vs.sumy.get());
+    enter_timing<M, V>(P, vs);
     std::vector<cudaEvent_t> ev(2 * iters + 1);
     for (auto& e : ev) GB_CUDA(cudaEventCreate(&e));
     long long nl = 0;
@@ -1995,6 +2009,43 @@ void time_level(Problem& P, int iters, double* msp, double* msd, int64_t* launch
     *launches = nl;
 }
 
+// Device time (ms) of what `body` launches, captured into a CUDA graph, in its
+// second run.
+template <class F>
+double timed_graph(cudaStream_t s, F&& body) {
+    cudaStream_t cs;
+    GB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t ge = nullptr;
+    GB_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    try {
+        body(cs);
+    } catch (...) {
+        cudaStreamEndCapture(cs, &g);
+        cudaGetLastError();
+        cudaStreamDestroy(cs);
+        throw;
+    }
+    GB_CUDA(cudaStreamEndCapture(cs, &g));
+    GB_CUDA(cudaStreamDestroy(cs));
+    GB_CUDA(cudaGraphInstantiate(&ge, g, 0));
+    cudaEvent_t e0, e1;
+    GB_CUDA(cudaEventCreate(&e0));
+    GB_CUDA(cudaEventCreate(&e1));
+    GB_CUDA(cudaGraphLaunch(ge, s));  // warm-up
+    GB_CUDA(cudaEventRecord(e0, s));
+    GB_CUDA(cudaGraphLaunch(ge, s));
+    GB_CUDA(cudaEventRecord(e1, s));
+    GB_CUDA(cudaEventSynchronize(e1));
+    float ms = 0;
+    GB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    cudaGraphExecDestroy(ge);
+    cudaGraphDestroy(g);
+    return static_cast<double>(ms);
+}
+
 // Average device time of k_primal and of k_dual when launched back to back
 // (each captured `iters` times into a CUDA graph with programmatic dependent
 // launch, as the solve loop issues them, and the graph timed with two CUDA
@@ -2005,59 +2056,50 @@ template <class M, class V>
 void time_level_graph(Problem& P, int iters, double* msp, double* msd, double* msi) {
     cudaStream_t s = P.stream;
     VecSet<V>& vs = Level<M, V>::vs(P);
-    k_activate_all<<<div_up(P.count, kThreads), kThreads, 0, s>>>(P.count, P.st.get());
-    k_phase_in<V><<<elem_grid(std::max(P.n, P.m), P.sms), kThreads, 0, s>>>(
-        P.n, P.m, P.icol(), P.irow(), P.st.get(), P.x64.get(), P.y64.get(), P.x64.get(), P.y64.get(), 0,
-        vs.x0.get(), vs.y0.get(), vs.xr.get(), vs.yr.get(), vs.sumx.get(), vs.sumy.get());
+    enter_timing<M, V>(P, vs);
     PrimalArgs<M, V> pa;
     DualArgs<M, V> da;
     iteration_args<M, V>(P, vs, 0, pa, da);
-    auto timed_graph = [&](auto&& body) {
-        cudaStream_t cs;
-        GB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t ge = nullptr;
-        GB_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        try {
-            body(cs);
-        } catch (...) {
-            cudaStreamEndCapture(cs, &g);
-            cudaGetLastError();
-            cudaStreamDestroy(cs);
-            throw;
-        }
-        GB_CUDA(cudaStreamEndCapture(cs, &g));
-        GB_CUDA(cudaStreamDestroy(cs));
-        GB_CUDA(cudaGraphInstantiate(&ge, g, 0));
-        cudaEvent_t e0, e1;
-        GB_CUDA(cudaEventCreate(&e0));
-        GB_CUDA(cudaEventCreate(&e1));
-        GB_CUDA(cudaGraphLaunch(ge, s));  // warm-up
-        GB_CUDA(cudaEventRecord(e0, s));
-        GB_CUDA(cudaGraphLaunch(ge, s));
-        GB_CUDA(cudaEventRecord(e1, s));
-        GB_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        GB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        cudaGraphExecDestroy(ge);
-        cudaGraphDestroy(g);
-        return static_cast<double>(ms) / iters;
-    };
     if (msp)
-        *msp = timed_graph([&](cudaStream_t cs) {
+        *msp = timed_graph(s, [&](cudaStream_t cs) {
             for (int k = 0; k < iters; ++k) launch_primal<M, V>(pa, cs);
-        });
+        }) / iters;
     if (msd)
-        *msd = timed_graph([&](cudaStream_t cs) {
+        *msd = timed_graph(s, [&](cudaStream_t cs) {
             for (int k = 0; k < iters; ++k) launch_dual<M, V>(da, cs);
-        });
-    *msi = timed_graph([&](cudaStream_t cs) {
+        }) / iters;
+    *msi = timed_graph(s, [&](cudaStream_t cs) {
         long long nl = 0;
         for (int k = 0; k < iters; ++k) launch_iteration<M, V>(P, vs, k, cs, nl);
+    }) / iters;
+    GB_CUDA(cudaGetLastError());
+}
+
+// Whether the solves of level <M, V> iterate on chip alone, and whether any
+// part of them does (prepare_resident ran).
+template <class M, class V>
+bool wholly_on_chip(const Problem& P) {
+    const ResPlan& R = P.res[sizeof(V) == 8];
+    return (R.any() && R.list_na[sizeof(M) == 8] == 0) || P.grid[sizeof(V) == 8].on || qp_on_chip<M, V>(P);
+}
+template <class M, class V>
+bool partly_on_chip(const Problem& P) {
+    return P.res[sizeof(V) == 8].any() || wholly_on_chip<M, V>(P);
+}
+
+// Average device time (ms) of an iteration as the body of a solve runs it, on
+// chip and streamed, every instance active.
+template <class M, class V>
+double time_body(Problem& P, int iters) {
+    VecSet<V>& vs = Level<M, V>::vs(P);
+    prepare_resident<M, V>(P);
+    enter_timing<M, V>(P, vs);
+    const double ms = timed_graph(P.stream, [&](cudaStream_t cs) {
+        long long nl = 0;
+        launch_iterations<M, V>(P, vs, iters, cs, nl);
     });
     GB_CUDA(cudaGetLastError());
+    return ms / iters;
 }
 
 template <class F>
@@ -2104,9 +2146,10 @@ void rebuild_schedules(Problem& P, int w) {
 // every candidate (block_nnz, max_rows) -- block_nnz bounds the nonzeros a
 // STREAM block stages (<= kBlockNnz, the shared-memory product buffer),
 // max_rows the rows it reduces and hence the lanes per row -- is tried with
-// the other classes at their incumbents, by timing `iters` fused iterations
-// (CUDA events around k_primal + k_dual), and kept when it is more than 1%
-// faster.  The per-row group size inside a block still follows the block's
+// the other classes at their incumbents, by timing iterations as a solve's body
+// runs them (`iters` at least; instances on chip on chip: a cut that makes their
+// longer rows LONG would push them off it), and kept when it is more than 1%
+// faster.  A class whose solves run wholly on chip keeps the default cut.  The per-row group size inside a block still follows the block's
 // row count (the row-length histogram).  Besides a fixed grid of candidates,
 // block sizes that cut the nonzeros into whole waves of resident CTAs are
 // tried: a launch of 1.2 waves leaves most SMs idle during its second wave.
@@ -2126,16 +2169,6 @@ void autotune_class(Problem& P, int w, int iters, double* ms_default, double* ms
         b = (b + 31) / 32 * 32;
         if (b >= 256 && b <= kBlockNnz) cand.push_back({static_cast<int>(b), kThreads});
     }
-    auto measure = [&]() {  // ms per iteration, back to back in a CUDA graph as the solve loop issues them
-        double best = INFINITY;
-        for (int rep = 0; rep < 2; ++rep) {
-            double mi = 0;
-            if (w == 0) time_level_graph<float, float>(P, iters, nullptr, nullptr, &mi);
-            else time_level_graph<double, double>(P, iters, nullptr, nullptr, &mi);
-            best = std::min(best, mi);
-        }
-        return best;
-    };
     auto& tb = P.tune_block_nnz[w];
     auto& tr = P.tune_max_rows[w];
     tb.assign(P.count, kBlockNnz);
@@ -2143,8 +2176,22 @@ void autotune_class(Problem& P, int w, int iters, double* ms_default, double* ms
     P.A.stream_nc[w] = P.A.default_nc[w];
     P.AT.stream_nc[w] = P.AT.default_nc[w];
     rebuild_schedules(P, w);
+    if (w == 0) prepare_resident<float, float>(P);
+    else prepare_resident<double, double>(P);
+    // an on-chip launch runs a whole check period
+    const int body = (w == 0 ? partly_on_chip<float, float>(P) : partly_on_chip<double, double>(P)) ? std::max(iters, 64) : iters;
+    auto measure = [&]() {  // ms per iteration, back to back in a CUDA graph as the solve loop issues them
+        double best = INFINITY;
+        for (int rep = 0; rep < 2; ++rep)
+            best = std::min(best, w == 0 ? time_body<float, float>(P, body) : time_body<double, double>(P, body));
+        return best;
+    };
     double best = measure();
     if (ms_default) *ms_default = best;
+    if (w == 0 ? wholly_on_chip<float, float>(P) : wholly_on_chip<double, double>(P)) {  // no streaming kernel to tune
+        if (ms_tuned) *ms_tuned = best;
+        return;
+    }
     // load mode of each matrix's kernel (k_dual reads A, k_primal A^T), the
     // other at its incumbent
     for (DevMat* mat : {&P.A, &P.AT}) {

@@ -180,7 +180,8 @@ void* gb_problem_stream(gb_problem* p);
  * runs `iters` plain PDHG iterations from the current iterate with CUDA
  * events around every launch and reports the mean duration (ms) of the fused
  * primal kernel (A^T y + primal step) and of the fused dual kernel (A xbar +
- * dual step), and the number of launches issued. */
+ * dual step), and the number of launches issued: the streaming kernels, also
+ * for a problem whose solves iterate on chip. */
 int gb_problem_time_kernels(gb_problem* p, int level, int iters, double* ms_primal, double* ms_dual,
                             int64_t* launches);
 /* Counters of the last gb_problem_solve: kernel launches issued inside the
@@ -198,7 +199,9 @@ int gb_problem_time_kernels_graph(gb_problem* p, int level, int iters, double* m
  * gb_batch_autotune): after a first solve, times candidate (block_nnz,
  * max_rows) cuts of the CSR row blocks -- including cuts into whole waves of
  * resident CTAs -- separately for the FP32/BF16-matrix kernels and the FP64
- * ones, and keeps the fastest of each.  Outputs are pairs [FP32, FP64]
+ * ones, and keeps the fastest of each.  What is timed is an iteration as a
+ * solve runs it; a level whose solves iterate on chip keeps the default cut.
+ * Outputs are pairs [FP32, FP64]
  * (block_nnz[2], max_rows[2], ms_default[2], ms_tuned[2]; any may be NULL).
  * Results stay certified; only the summation grouping inside a row changes. */
 int gb_problem_autotune(gb_problem* p, int iters, int* block_nnz, int* max_rows, double* ms_default,
@@ -318,11 +321,13 @@ int gb_batch_get_solutions(gb_batch* b, double* x_out, double* y_out);
 int gb_batch_schedule(gb_batch* b, int* threads, int* blocks_per_sm, int* groups);
 /* Row-split schedule autotuner: per class of instance sizes (four classes of
  * equal total nonzeros), picks (block_nnz, max_rows) of the CSR row blocks by
- * timing `iters` fused iterations per candidate with CUDA events -- once for
- * the schedule of the FP32/BF16-matrix kernels (timed at FP32), once for that
- * of the FP64 kernels (timed at FP64).  Writes the chosen values per instance
- * (arrays of 2 * count: FP32 schedule then FP64; may be NULL) and the
- * per-iteration kernel time of the default and tuned schedules (ms, [2]). */
+ * timing `iters` iterations (at least) per candidate with CUDA events, as a
+ * solve runs them, on chip and streamed -- once for the schedule of the
+ * FP32/BF16-matrix kernels (timed at FP32), once for that of the FP64 kernels
+ * (timed at FP64); a level whose solves run wholly on chip keeps the default
+ * cut.  Writes the chosen values per instance (arrays of 2 * count: FP32
+ * schedule then FP64; may be NULL) and the time of an iteration with the
+ * default and tuned schedules (ms, [2]). */
 int gb_batch_autotune(gb_batch* b, int iters, int* block_nnz, int* max_rows, double* ms_default, double* ms_tuned);
 /* Load variant of the fused iteration kernels, per matrix and precision
  * class: modes[0..3] = A (FP32/BF16 kernels), A^T (FP32/BF16), A (FP64),
