@@ -1075,6 +1075,9 @@ struct Diff {
             auto kernel = rows <= kMrSolveThreads ? k_mr_solve_chip<1> : k_mr_solve_chip<2>;
             GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMrChipSmem)));
             kernel<<<p.count, kMrSolveThreads, chip.bytes(), s>>>(oa, chip);
+            if (trace_enabled())
+                std::fprintf(stderr, "[gb trace] minres on chip: %d rows, %d a thread, %zu B\n", rows,
+                             rows <= kMrSolveThreads ? 1 : 2, chip.bytes());
         } else if (one_launch) {
             k_mr_solve<<<p.count, kMrSolveThreads, 0, s>>>(oa);
         } else if (host_loop_mode()) {  // the same steps from the host, one state read-back per chunk

@@ -1132,6 +1132,9 @@ void launch_qp_chip(Problem& P, VecSet<V>& vs, int ce, cudaStream_t s) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     GB_CUDA(cudaLaunchKernelEx(&cfg, k_qp_chip<M, V>, a));
+    if (trace_enabled())
+        std::fprintf(stderr, "[gb trace] qp on chip f%d/f%d: %d of %d columns a slice in shared memory\n",
+                     sizeof(M) == 8 ? 64 : 32, sizeof(V) == 8 ? 64 : 32, a.smem_rows, a.rows_per);
 }
 
 // The FP64 plan, ahead of the power iteration that runs on it.
