@@ -627,6 +627,9 @@ class BatchSolver:
         return len(self.lps)
 
     def solve(self, opt: Options | None = None, fetch: bool = True) -> list:
+        """Results in the order of the LPs.  Their ``x`` and ``y`` are parts of one
+        array each, which stays alive as long as any of them is kept: copy a
+        point that should outlive the others' memory."""
         o = _opts(opt)
         res = (_GbResult * len(self.lps))()
         _check(self._lib.gb_batch_solve(self._h, C.addressof(o), res))
