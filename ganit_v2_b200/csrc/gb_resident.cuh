@@ -186,6 +186,17 @@ __device__ __forceinline__ bool cluster_exchange(const void* p, unsigned bytes, 
     return lost || !mbar_wait(bar, parity);
 }
 
+// End of a CTA's work: it does not leave while a copy may still read its share.
+// Copies to it are in, since it awaited them, unless a wait ran out: then it
+// stays for about a millisecond after every CTA has sent its last (a copy takes
+// microseconds).
+__device__ __forceinline__ void cluster_leave(int cluster, bool lost) {
+    if (cluster == 1) return;
+    cluster_sync();
+    if (lost)
+        for (int k = 0; k < 64; ++k) __nanosleep(16000);
+}
+
 // Two matrix values of a lane's step pair.
 __device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
     const float2 v = *reinterpret_cast<const float2*>(p);
@@ -425,7 +436,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_resident(const __grid_c
         a.y[i] = ys[r.pos_a0 + k];
         a.sumy[i] = osy[k];
     }
-    if (a.cluster > 1) cluster_sync();  // no CTA leaves while a copy may still read its share
+    cluster_leave(a.cluster, lost);
 }
 
 // Power iteration on A'^T A' (scaling.cpp:131-155) of the resident instances on
@@ -522,7 +533,7 @@ __global__ void __launch_bounds__(T, T < 1024 ? 2 : 1) k_power_chip(const __grid
     }
     if (lost && tid == 0) atomicExch(a.error, 1);
     if (rank == 0 && tid == 0) a.scal[static_cast<size_t>(r.inst) * a.scal_stride + a.lambda] = lambda;
-    if (a.cluster > 1) cluster_sync();
+    cluster_leave(a.cluster, lost);
 }
 
 // ---------------------------------------------------------------- packing (device, once per plan)
