@@ -324,6 +324,7 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     if (count > 1)
         for (int k = 0; k < count; ++k)
             GB_REQUIRE(lps[k].q_ptr == nullptr && lps[k].q_rank == 0, "batched solving takes LPs only (no Hessian)");
+    FreeBatchEnd set_up;  // outlives the set-up's buffers
     auto P = std::make_unique<Problem>();
     P->device = g_device;
     GB_CUDA(cudaSetDevice(P->device));
@@ -561,6 +562,8 @@ Problem* create_problem(int count, const gb_lp* lps, const gb_options* opt) {
     GB_CUDA(cudaStreamSynchronize(s));
     GB_CUDA(cudaGetLastError());
     if (P->phase_flags_host[count]) throw Error(GB_ERR_CUDA, "an exchange between the CTAs of a cluster timed out");
+    begin_free_batch();  // one device synchronisation for all that set-up gives back
+    set_up.open = true;
     release_plan_scratch(*P);
     P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return P.release();
