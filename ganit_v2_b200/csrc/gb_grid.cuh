@@ -2,8 +2,8 @@
 // keeps it, one CTA per SM, a check period per cooperative launch.
 //
 // The streaming kernels take two dependent launches and a pass over the matrix
-// in L2 per iteration: 13.6 us on a blending LP of 411K nonzeros in FP64,
-// 16.6 us at 2.9M in FP32.  Here every CTA owns a contiguous share of A^T's
+// in L2 per iteration: 13.7 us on a blending LP of 411K nonzeros in FP64,
+// 17.0 us at 2.9M in FP32.  Here every CTA owns a contiguous share of A^T's
 // rows and of A's rows (by nonzeros) with its matrix entries, vectors and
 // iterate in shared memory.  The entries of y and xbar that its rows gather --
 // for an LP with any locality a small part -- are listed once; every half
@@ -21,10 +21,12 @@
 //
 // What bounds it: two trips through L2 per iteration at small sizes; at 2.9M
 // nonzeros the shared-memory wavefronts of the sums and the 40 % of the matrix
-// that comes from L2.  Measured on B200, us an iteration, streaming -> with two
-// grid barriers an iteration -> with tags: blending 120K nonzeros FP64 9.2 -> 6.2
-// -> 4.3, 411K FP64 14.6 -> 7.1 -> 5.7, 2.9M FP32 18.7 -> 13.2 -> 11.9; random
-// 6000 x 15001 (no locality) FP64 10.4 -> 7.3 -> 7.5, FP32 9.5 -> 7.2 -> 7.4.
+// that comes from L2.  Measured on B200, us an iteration of solves of 2,048
+// iterations, checks included, streaming -> here: blending 120K nonzeros FP64
+// 8.7 -> 4.0, 411K FP64 13.7 -> 4.8, 2.9M FP32 17.0 -> 10.0; random 6000 x 15001
+// (no locality) FP64 9.5 -> 5.7, FP32 7.7 -> 5.9.  With two grid barriers an
+// iteration in place of the tags the three blending LPs took 1.44, 1.25 and 1.11
+// times as long, the random one 0.97 times.
 #pragma once
 #include "gb_qp_chip.cuh"
 #include "gb_resident.cuh"

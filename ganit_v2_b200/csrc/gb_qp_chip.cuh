@@ -30,13 +30,14 @@
 // of F from shared memory and their FP64 chains (13 K), then three trips of the
 // words through L2.  8,009 x 33 is the trips alone: 9 % of the shared-memory
 // wavefronts, warps waiting for words.
-// Measured on B200, streaming -> here: 100,000 x 50 FP64 29 -> 11.7 us an
-// iteration, 8,009 x 33 mixed 18.5 -> 6.0 us.  With two grid barriers an
-// iteration in place of the tags it was 12.7 and 7.0 us; with the last arrival
-// of a chunk running the dual step, and x and bounds read behind the barrier,
-// 16 and 10 us.  Reading F once (a warp per four columns, partials by
-// transposing shuffles) took 20.4 and 7.0 us against 14.5 and 8.1 at that
-// point: the shuffles cost more than the second read saves.
+// Measured on B200, us an iteration of solves of 2,048 iterations, checks
+// included, streaming -> here: 100,000 x 50 FP64 32.8 -> 12.4, 8,009 x 33 mixed
+// 18.5 -> 6.7.  Of the iterations alone (11.7 and 6.0 us): with two grid barriers
+// an iteration in place of the tags 12.7 and 7.0; with the last arrival of a chunk
+// running the dual step, and x and bounds read behind the barrier, 16 and 10.
+// Reading F once (a warp per four columns, partials by transposing shuffles) took
+// 20.4 and 7.0 us against 14.5 and 8.1 at that point: the shuffles cost more than
+// the second read saves.
 #pragma once
 #include "gb_qp.cuh"
 #include "gb_resident.cuh"
