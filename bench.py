@@ -23,7 +23,8 @@ time = max over ranks).
 
 ``--impl reference`` times the reference's own CPU implementation
 (ganit::solve_pdhg_cpu, oracle/_ref/libganit_ref.so built from the reference
-sources) with all host threads, on rank 0 only.  The default arm also times
+sources) with all host threads, on rank 0 only; without that build it says so
+and times nothing.  The default arm also times
 the reference's own CUDA backend (ganit::solve_pdhg_gpu, built unmodified for
 sm_100a into oracle/_ref/libganit_refcuda.so) on the same LP and GPU
 (``reference_cuda``).
@@ -168,9 +169,13 @@ def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
-    lp = workload()
     from oracle import oracle as O
 
+    if not O.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libganit_ref.so not built: it needs the "
+                          "reference's sources, which have no installable package"}), flush=True)
+        return 0
+    lp = workload()
     for _ in range(args.warmup):
         cpu_baseline_run(lp, 1)
     vals, kind, cores, secs, res = None, None, None, [], None
@@ -182,7 +187,7 @@ def run_reference_arm(args):
         "impl": "reference", "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": args.gpus,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * sum(secs) / len(secs),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",
-        "config": dict(CONFIG), "parallelism": "cpu-openmp" if kind == "reference" else "cpu-1-thread",
+        "config": dict(CONFIG), "parallelism": "cpu-openmp",
         "cpu_baseline": {"value": value, "unit": UNIT, "cores": cores, "kind": kind,
                          "sample": f"{args.steps} full mixed-precision solves of the blending LP "
                                    f"({res.iterations} iterations, status {res.status})"},
