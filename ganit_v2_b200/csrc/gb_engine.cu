@@ -2128,9 +2128,15 @@ void rebuild_schedules(Problem& P, int w) {
     GB_CUDA(cudaStreamSynchronize(s));
     release_plan_scratch(P);
     for (auto& g : P.graphs) g.reset();
-    for (ResPlan& r : P.res) r = ResPlan{};  // packed by these schedules' lanes per row
-    for (GridPlan& r : P.grid) r = GridPlan{};
-    P.qp_at_lg.release();
+    // plans follow the schedule of their vector type (lanes per row), the FP64
+    // plan's streamed lists that of the FP32 matrix too
+    P.res[1] = ResPlan{};
+    P.grid[1] = GridPlan{};
+    if (w == 0 || P.A.sched32.nb == 0) {
+        P.res[0] = ResPlan{};
+        P.grid[0] = GridPlan{};
+        P.qp_at_lg.release();
+    }
     DevSchedule& sa = w == 0 ? P.A.sched32 : P.A.sched;
     DevSchedule& st = w == 0 ? P.AT.sched32 : P.AT.sched;
     sa.upload(build_schedule(P.A.host_ptr.data(), P.row_off.data(), P.count, P.tune_block_nnz[w].data(),
@@ -2253,7 +2259,8 @@ void autotune_class(Problem& P, int w, int iters, double* ms_default, double* ms
         }
     }
     rebuild_schedules(P, w);
-    if (ms_tuned) *ms_tuned = measure();
+    best = measure();  // also makes the plan that the next solve runs on
+    if (ms_tuned) *ms_tuned = best;
 }
 
 // Both classes; outputs [FP32, FP64].
